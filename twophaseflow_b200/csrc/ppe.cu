@@ -804,22 +804,20 @@ __global__ void __launch_bounds__(kThreads, 1) cg1_batch_kernel(const __grid_con
   cg1_body<T, MIXED>(b.c[c], blockIdx.x - b.first[c], b.first[c + 1] - b.first[c]);
 }
 
-// ---- band-resident PCG (2-D; FP64, or FP32 under FP64 residual replacement) ----------------
+// ---- band-resident PCG (2-D) ---------------------------------------------------------------
 //
 // The same Chronopoulos-Gear iteration as cg1_body (Jacobi or none), for 2-D
-// systems whose per-SM share fits in shared memory (513^2 on 148 SMs:
-// ~1 780 nodes per SM in FP64, twice that in FP32).  CTA b owns the
-// contiguous node range [b ndof / G, (b+1) ndof / G) (balanced to one node;
-// every range is at least one row of W = n1 nodes long); its r, w, s
-// (double-buffered), p, x, M^-1 and both face couplings stay in shared memory
-// for the whole solve.  The stencil reaches W nodes back and forward, which
-// lie in the two adjacent ranges: each CTA publishes its first and last W
-// nodes' (r, w, s) before the barrier (double-buffered by iteration parity; a
-// slot is rewritten only after its readers have arrived at the next barrier)
-// and reads its neighbours' after it.  Per iteration: u = M r once per node
+// systems whose per-SM share stays on the SM for the whole solve.  CTA b owns
+// the contiguous node range [b ndof / G, (b+1) ndof / G) (balanced to one
+// node; every range is at least one row of W = n1 nodes long).  The stencil
+// reaches W nodes back and forward, which lie in the two adjacent ranges: each
+// CTA publishes its first and last W nodes (double-buffered by iteration
+// parity) and reads its neighbours'.  Per iteration: u = M r once per node
 // (sub-pass 1), w = S u from shared memory (sub-pass 2), one grid-wide
-// reduction; x is written back once at the end, so the only global traffic
-// of an iteration is the halo and the reduction.
+// reduction; x is written back once at the end, so the only global traffic of
+// an iteration is the halo and the reduction.  FP64 systems keep their vectors in registers
+// (cg1_band_reg_body); FP32 systems under FP64 residual replacement keep them
+// in shared memory (cg1_band_mixed_body).
 //
 // Layout: u is stored as [W nodes before the range | the range | W nodes
 // after it] and the couplings as [W nodes before | the range], so every
@@ -831,46 +829,179 @@ __global__ void __launch_bounds__(kThreads, 1) cg1_batch_kernel(const __grid_con
 // s_row does.  The pin node's u is stored as 0 (its column is zero); its own
 // u is recomputed where its row needs it.
 //
-// MIXED (T = float): the vectors, couplings and M^-1 are FP32, x and the
-// inner products FP64, and the residual is replaced by the FP64 b - S x
-// (couplings from the FP64 arrays in global memory, the neighbours' x edges
-// published through global memory) whenever ||r|| has fallen by
-// replace_drop since the last replacement and before accepting convergence,
-// followed by a CG restart -- the rule of cg1_body<float, true>.
+// Mixed: the vectors, couplings and M^-1 are FP32, x and the inner products
+// FP64, and the residual is replaced by the FP64 b - S x (couplings from the
+// FP64 arrays in global memory, the neighbours' x edges published through
+// global memory) whenever ||r|| has fallen by replace_drop since the last
+// replacement and before accepting convergence, followed by a CG restart --
+// the rule of cg1_body<float, true>.
+
+// A double that travels between blocks of one launch as a 16-byte slot of two
+// 8-byte words, each half the value and the epoch: a reader that finds the
+// epoch in both words has the value, so nothing else orders writer and reader
+// (no fence, no counter).
+struct __align__(16) FlagSlot {
+  unsigned long long lo, hi;
+};
+__device__ __forceinline__ void slot_store(FlagSlot* p, double v, unsigned int tag) {
+  const unsigned long long x = (unsigned long long)__double_as_longlong(v), t = (unsigned long long)tag << 32;
+  asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"((x & 0xffffffffull) | t),
+               "l"((x >> 32) | t)
+               : "memory");
+}
+// The words of slot p if `want`, untouched otherwise: a predicated load rather
+// than a branch, so that the polls of several slots are in flight together.
+__device__ __forceinline__ void slot_load(const FlagSlot* p, bool want, FlagSlot& q) {
+  asm volatile("{\n .reg .pred w;\n setp.ne.u32 w, %3, 0;\n @w ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];\n}"
+               : "+l"(q.lo), "+l"(q.hi)
+               : "l"(p), "r"((unsigned int)want)
+               : "memory");
+}
+__device__ __forceinline__ bool slot_ready(const FlagSlot& q, unsigned int tag) {
+  return (unsigned int)(q.lo >> 32) == tag && (unsigned int)(q.hi >> 32) == tag;
+}
+__device__ __forceinline__ double slot_value(const FlagSlot& q) {
+  return __longlong_as_double((long long)((q.lo & 0xffffffffull) | (q.hi << 32)));
+}
+
+constexpr int kBandThreads = 256;    // threads of the FP64 kernel
+constexpr int kBandWarps = kBandThreads / 32;
+constexpr int kBandSums = 6;         // inner products of an iteration
+constexpr int kBandLine = 8;         // slots per block: its sums, padded to one 128-byte line
+constexpr int kBandPoll = 6;         // groups of four blocks per polling warp
+constexpr int kBandMaxGrid = 4 * kBandWarps * kBandPoll;   // 192 blocks of one system
+constexpr int kBandMaxW = 768;       // nodes of a row
+constexpr int kBandHalo = 2 * kBandMaxW / kBandThreads;    // halo entries per thread
+
+// Totals of kBandSums values over the blocks [0, G) of one system: the
+// block's sums go out as slots of this epoch, every block polls the slots of
+// all blocks (bounded) and adds them in a fixed order, so every block has the
+// same bits.  The values edge_v[2 W] (shared memory) of the range's first and
+// last W nodes go out too, and the halo slots edges + hoff[e] (e < kBandHalo,
+// hoff < 0: none) are polled in the same wait.  On success `then(totals)` runs
+// in thread 0 and is visible to the block on return.  Slots alternate between two sets by epoch parity; a block
+// rewrites a set only after it has seen every block's slots of the epoch
+// between, i.e. after every block has read it.
+//
+// A block's slots fill a line of their own: with the six values of all blocks
+// side by side instead (eight writers to a line) the same exchange took 4.6 us
+// over 148 blocks against 1.5 us.
+template <typename Then>
+__device__ __forceinline__ bool band_exchange(FlagSlot* slots, FlagSlot* edges, int* err, const int G, const int bid,
+                                              const unsigned int tag, const double (&v)[kBandSums],
+                                              const double* edge_v, const int W, const int (&hoff)[kBandHalo],
+                                              double (&hv)[kBandHalo], Then&& then) {
+  __shared__ double own[kBandSums * kBandWarps], part[kBandSums * kBandWarps], tot[kBandSums];
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+  const unsigned m = 0xffffffffu;
+  static_assert(kBandSums == 6 && kBandWarps == 8, "the sums below are written out for 6 values and 8 warps");
+  {
+    // six warp sums in nine shuffles: each of the first three steps halves the
+    // values a lane carries; lane 4 k ends with value k
+    const bool h16 = lane & 16, h8 = lane & 8, h4 = lane & 4;
+    const double x0 = (h16 ? v[4] : v[0]) + __shfl_xor_sync(m, h16 ? v[0] : v[4], 16);
+    const double x1 = (h16 ? v[5] : v[1]) + __shfl_xor_sync(m, h16 ? v[1] : v[5], 16);
+    const double x2 = (h16 ? 0.0 : v[2]) + __shfl_xor_sync(m, h16 ? v[2] : 0.0, 16);
+    const double x3 = (h16 ? 0.0 : v[3]) + __shfl_xor_sync(m, h16 ? v[3] : 0.0, 16);
+    const double y0 = (h8 ? x2 : x0) + __shfl_xor_sync(m, h8 ? x0 : x2, 8);
+    const double y1 = (h8 ? x3 : x1) + __shfl_xor_sync(m, h8 ? x1 : x3, 8);
+    double z = (h4 ? y1 : y0) + __shfl_xor_sync(m, h4 ? y0 : y1, 4);
+    z += __shfl_xor_sync(m, z, 2);
+    z += __shfl_xor_sync(m, z, 1);
+    if ((lane & 3) == 0 && (lane >> 2) < kBandSums) own[(lane >> 2) * kBandWarps + wid] = z;
+  }
+  auto sum8 = [](const double* p) { return ((p[0] + p[1]) + (p[2] + p[3])) + ((p[4] + p[5]) + (p[6] + p[7])); };
+  __syncthreads();
+  if (t < kBandSums) slot_store(slots + (size_t)bid * kBandLine + t, sum8(own + t * kBandWarps), tag);
+#pragma unroll
+  for (int e = 0; e < kBandHalo; ++e) {
+    const int k = t + e * kBandThreads;
+    if (k < 2 * W) slot_store(edges + (size_t)bid * 2 * W + k, edge_v[k], tag);
+  }
+  // poll: warp w the blocks 4 (w + 8 j) + lane / 8, lane % 8 the value
+  FlagSlot qs[kBandPoll], qh[kBandHalo];
+  unsigned need = 0;
+#pragma unroll
+  for (int j = 0; j < kBandPoll; ++j) {
+    qs[j] = {0, 0};
+    if ((lane & (kBandLine - 1)) < kBandSums && 4 * (wid + kBandWarps * j) + lane / kBandLine < G) need |= 1u << j;
+  }
+#pragma unroll
+  for (int e = 0; e < kBandHalo; ++e) {
+    qh[e] = {0, 0};
+    if (hoff[e] >= 0) need |= 256u << e;
+  }
+  bool ok = true;
+  const FlagSlot* mine = slots + 32 * wid + lane;
+  for (long long spins = 0; need;) {
+#pragma unroll
+    for (int j = 0; j < kBandPoll; ++j) slot_load(mine + 32 * kBandWarps * j, need & (1u << j), qs[j]);
+#pragma unroll
+    for (int e = 0; e < kBandHalo; ++e) slot_load(edges + hoff[e], need & (256u << e), qh[e]);
+#pragma unroll
+    for (int j = 0; j < kBandPoll; ++j)
+      if (slot_ready(qs[j], tag)) need &= ~(1u << j);
+#pragma unroll
+    for (int e = 0; e < kBandHalo; ++e)
+      if (slot_ready(qh[e], tag)) need &= ~(256u << e);
+    if (++spins > kSpinLimit) { atomicExch(err, 1); ok = false; break; }
+    if ((spins & 1023) == 0 && *(volatile int*)err) { ok = false; break; }
+  }
+  __syncwarp();
+  double val[kBandPoll];
+#pragma unroll
+  for (int j = 0; j < kBandPoll; ++j) val[j] = slot_value(qs[j]);   // a slot not asked for reads as 0
+#pragma unroll
+  for (int e = 0; e < kBandHalo; ++e) hv[e] = slot_value(qh[e]);
+  double z = ((val[0] + val[1]) + (val[2] + val[3])) + (val[4] + val[5]);
+  z += __shfl_xor_sync(m, z, 8);
+  z += __shfl_xor_sync(m, z, 16);
+  if (lane < kBandSums) part[lane * kBandWarps + wid] = z;
+  ok = __syncthreads_and(ok) != 0;
+  if (ok && wid == 0) {
+    if (lane < kBandSums) tot[lane] = sum8(part + lane * kBandWarps);
+    __syncwarp();
+    if (lane == 0) then(tot);
+  }
+  __syncthreads();
+  return ok;
+}
+
 struct BandArgs {
   Grid3 g;
   const double* s0;      // couplings to the next row (axis 0), 0 on the last row
   const double* s1;      // couplings to the next column (axis 1), 0 on the last column
   const double* dinv;    // Jacobi 1/diag(S) (pin -> 1), or ones
-  const float* s0f;      // FP32 copies (MIXED)
+  const float* s0f;      // FP32 copies (mixed)
   const float* s1f;
   const float* dinvf;
   const double* b;       // SPD-system rhs
   double* x;             // solution
   long long maxiter;
   double tol;
-  double replace_drop;   // MIXED: replace the residual when ||r|| fell by this factor
+  double replace_drop;   // mixed: replace the residual when ||r|| fell by this factor
   int x_nonzero;
   int n_max;             // nodes of the largest range
-  void* pub;             // [2 parity][G][2 side: first / last W nodes][3 vec: r, w, s][W] of T
-  double* part;          // [2 slots][8][G]
-  unsigned int* count;   // monotonic arrival counter
+  FlagSlot* slots;       // FP64: [2 parity][G][kBandLine] sums, then [2 parity][G][2 side: first / last W
+                         // nodes][W] edges; tags zeroed before the launch
+  float* pub;            // mixed: [2 parity][G][2 side][3 vec: r, w, s][W]
+  double* part;          // mixed: [2 slots][8][G]
+  unsigned int* count;   // mixed: monotonic arrival counter
   int* err;
   SolveStatus* st;
 };
 
-// shared-memory bytes: x (FP64) + 11 range arrays of T + 6 rows of halo of T
-// (u 2, couplings 2, M^-1 2)
-template <typename T>
-inline size_t band_smem_bytes(int n_max, int n1) {
-  return (size_t)n_max * sizeof(double) + ((size_t)11 * n_max + 6 * (size_t)n1) * sizeof(T);
+// shared-memory bytes of the mixed body: x (FP64) + 11 FP32 range arrays + 6
+// FP32 rows of halo (u 2, couplings 2, M^-1 2)
+inline size_t band_mixed_smem_bytes(int n_max, int n1) {
+  return (size_t)n_max * sizeof(double) + ((size_t)11 * n_max + 6 * (size_t)n1) * sizeof(float);
 }
 
-// The whole band-resident solve of one system by blocks [0, G) of a grid
+// The whole mixed-precision solve of one system by blocks [0, G) of a grid
 // (bid = this block's index): the full grid for a single solve, or one
 // case's share of a batched launch.
-template <typename T, bool MIXED>
-__device__ __forceinline__ void cg1_band_body(const BandArgs& a, const int bid, const int G) {
+__device__ __forceinline__ void cg1_band_mixed_body(const BandArgs& a, const int bid, const int G) {
+  using T = float;
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ double scratch[256];
   const Grid3& g = a.g;
@@ -890,15 +1021,10 @@ __device__ __forceinline__ void cg1_band_body(const BandArgs& a, const int bid, 
   T* A1e = A0e + NM + W;          // [W before | range]            (NM + W)
   T* HD = A1e + NM + W;           // [2][W]: M^-1 of the nodes before / after the range
   T* Ua = Ue + W + nown;          // u of the W nodes after the range
-  const T* s0t;
-  const T* s1t;
-  const T* dit;
-  if constexpr (MIXED) {
-    s0t = a.s0f; s1t = a.s1f; dit = a.dinvf;
-  } else {
-    s0t = a.s0; s1t = a.s1; dit = a.dinv;
-  }
-  T* const pubv = static_cast<T*>(a.pub);
+  const T* s0t = a.s0f;
+  const T* s1t = a.s1f;
+  const T* dit = a.dinvf;
+  T* const pubv = a.pub;
   const bool has_up = bid > 0, has_dn = bid < G - 1;
   GridSum gs{a.part, a.count, a.err, (unsigned int)G, 0u, (unsigned int)bid};
   auto pub = [&](int par, int blk, int side, int vec) -> T* {
@@ -917,7 +1043,7 @@ __device__ __forceinline__ void cg1_band_body(const BandArgs& a, const int bid, 
     return (side == 0 ? has_up : has_dn) && q >= 0 && q < g.ndof;
   };
   auto hslot = [&](int side, int k) -> T& { return side == 0 ? Ue[k] : Ua[k]; };
-  // FP64 (S x)_idx of own node o (MIXED): x of own nodes from shared memory,
+  // FP64 (S x)_idx of own node o: x of own nodes from shared memory,
   // of the neighbour ranges' edges from global memory, couplings FP64 from
   // global memory (0 on boundary faces; out-of-domain neighbours skipped)
   auto sx64 = [&](int o) -> double {
@@ -995,37 +1121,12 @@ __device__ __forceinline__ void cg1_band_body(const BandArgs& a, const int bid, 
   }
   __syncthreads();
 
-  // r0 = b - S x (pin column zero / pin row identity); FP64: x, pin zeroed,
-  // staged in Ue; MIXED: sx64 over the initial x in global memory
+  // r0 = b - S x (pin column zero / pin row identity) from the initial x
   double red0[2] = {0.0, 0.0};
-  if (!MIXED && a.x_nonzero) {
-    for (int o = t; o < nown; o += NT) Ue[W + o] = (base + o == g.pin) ? T(0) : (T)X[o];
-    for (int k = t; k < 2 * W; k += NT) {
-      const int side = k / W, kk = k - side * W;
-      const int q = hq(side, kk);
-      hslot(side, kk) = (hlive(side, kk) && q != g.pin) ? (T)a.x[q] : T(0);
-    }
-    __syncthreads();
-  }
   for (int o = t; o < nown; o += NT) {
-    const int idx = base + o;
-    const double bi = a.b[idx];
+    const double bi = a.b[base + o];
     double ri = bi;
-    if (a.x_nonzero) {
-      double sx;
-      if constexpr (MIXED) {
-        sx = sx64(o);
-      } else {
-        if (idx == g.pin) {
-          sx = X[o];
-        } else {
-          T d, off;
-          stencil(Ue, o, d, off);
-          sx = d * X[o] - off;
-        }
-      }
-      ri = bi - sx;
-    }
+    if (a.x_nonzero) ri = bi - sx64(o);
     rb[0][o] = (T)ri;
     red0[0] += bi * bi;
     red0[1] += ri * ri;
@@ -1050,48 +1151,43 @@ __device__ __forceinline__ void cg1_band_body(const BandArgs& a, const int bid, 
   bool ok = gs.sum<6>(red, scratch);
   double gamma = red[0], rr = red[5];
   double beta = 0.0, denom = red[1];
-  double rr_ref = rr;    // ||r||^2 at the last FP64 residual replacement (MIXED)
+  double rr_ref = rr;    // ||r||^2 at the last FP64 residual replacement
   long long it = 0, replacements = 0, applies = a.x_nonzero ? 2 : 1;
   bool conv = false;
   int cur = 0;
-  constexpr int KH = 3;   // halo entries per thread: 2 * W <= KH * kThreads
+  constexpr int KH = 2 * kBandMaxW / kThreads;   // halo entries per thread
   while (ok) {
-    if constexpr (MIXED) {
-      const bool small = rr < atol2;
-      if (!small && it >= a.maxiter) break;
-      if (small || rr < a.replace_drop * a.replace_drop * rr_ref) {
-        // publish the x edges, barrier, r = b - S x in FP64 (halo r at
-        // parity cur ^ 1), barrier with ||r||^2, then a CG restart
-        for (int o = t; o < nown; o += NT)
-          if (o < W || o >= nown - W) a.x[base + o] = X[o];
-        double bar1[1] = {0.0};
-        if (!(ok = gs.sum<1>(bar1, scratch))) break;
-        double rt[1] = {0.0};
-        for (int o = t; o < nown; o += NT) {
-          const double ri = a.b[base + o] - sx64(o);
-          rb[cur][o] = (T)ri;
-          rt[0] += ri * ri;
-          if (o < W) pub(cur ^ 1, bid, 0, 0)[o] = (T)ri;
-          if (o >= nown - W) pub(cur ^ 1, bid, 1, 0)[o - (nown - W)] = (T)ri;
-        }
-        ++replacements;
-        ++applies;
-        if (!(ok = gs.sum<1>(rt, scratch))) break;
-        if (rt[0] < atol2) { rr = rt[0]; conv = true; break; }
-        if (it >= a.maxiter) { rr = rt[0]; break; }
-        init_pass(cur, red);
-        ++applies;
-        if (!(ok = gs.sum<6>(red, scratch))) break;
-        beta = 0.0;
-        denom = red[1];
-        gamma = red[0];
-        rr = red[5];
-        rr_ref = rr;
-        continue;
+    const bool small = rr < atol2;
+    if (!small && it >= a.maxiter) break;
+    if (small || rr < a.replace_drop * a.replace_drop * rr_ref) {
+      // publish the x edges, barrier, r = b - S x in FP64 (halo r at
+      // parity cur ^ 1), barrier with ||r||^2, then a CG restart
+      for (int o = t; o < nown; o += NT)
+        if (o < W || o >= nown - W) a.x[base + o] = X[o];
+      double bar1[1] = {0.0};
+      if (!(ok = gs.sum<1>(bar1, scratch))) break;
+      double rt[1] = {0.0};
+      for (int o = t; o < nown; o += NT) {
+        const double ri = a.b[base + o] - sx64(o);
+        rb[cur][o] = (T)ri;
+        rt[0] += ri * ri;
+        if (o < W) pub(cur ^ 1, bid, 0, 0)[o] = (T)ri;
+        if (o >= nown - W) pub(cur ^ 1, bid, 1, 0)[o - (nown - W)] = (T)ri;
       }
-    } else {
-      if (rr < atol2) { conv = true; break; }
-      if (it >= a.maxiter) break;
+      ++replacements;
+      ++applies;
+      if (!(ok = gs.sum<1>(rt, scratch))) break;
+      if (rt[0] < atol2) { rr = rt[0]; conv = true; break; }
+      if (it >= a.maxiter) { rr = rt[0]; break; }
+      init_pass(cur, red);
+      ++applies;
+      if (!(ok = gs.sum<6>(red, scratch))) break;
+      beta = 0.0;
+      denom = red[1];
+      gamma = red[0];
+      rr = red[5];
+      rr_ref = rr;
+      continue;
     }
     const double alpha_d = gamma / denom;
     const T alpha = (T)alpha_d, bt = (T)beta;
@@ -1190,25 +1286,351 @@ __device__ __forceinline__ void cg1_band_body(const BandArgs& a, const int bid, 
   }
 }
 
-template <typename T, bool MIXED>
-__global__ void __launch_bounds__(kThreads, 1) cg1_band_kernel(BandArgs a) {
-  cg1_band_body<T, MIXED>(a, blockIdx.x, gridDim.x);
+
+// FP64 band-resident PCG: a thread keeps its nodes in registers -- r, w, s, p,
+// x, M^-1, u and the couplings -- and only u goes through shared memory.
+//
+// What bounds it: nothing of the iteration touches HBM, so the time is the
+// latency of one grid-wide exchange plus the block's own two sub-passes.  The
+// shared-memory form of this kernel took 7.0 us an iteration at 513^2: ~24
+// values per node through shared memory (1.4 us of wavefronts), a counter
+// barrier, a read of the partial sums and a read of the neighbours' edges,
+// each a dependent L2 round trip behind a fence.  Here the sums and the edges
+// travel as self-validating slots, polled together in one round trip without
+// any fence.  Only w of the edge nodes travels: the reader carries their r and
+// s itself by the same two recurrences (fused multiply-adds spelled out, so
+// both copies have the same bits).
+// 513^2 to 1e-8: 25.6 -> 11.6 ms, 3.0 us an iteration, of which ~1.5 us are
+// the exchange over 148 blocks alone.
+//
+// 256 threads of up to 255 registers rather than 512 of 128: the per-warp cost
+// of an iteration (the reduction's shuffles, the scalars, index arithmetic) is
+// issued by half as many warps, and the E nodes of a thread hide the FP64
+// latency.  Thread t owns the consecutive nodes t E .. t E + E - 1, so that the
+// two neighbours along the row mostly are its own registers; E is odd, which
+// keeps the E-strided shared-memory accesses free of bank conflicts.  Up to
+// E = 9 the couplings are in registers too (x from E = 9 on in shared memory);
+// E = 11 keeps them in shared memory.  E is the smallest that covers the
+// largest range, so small systems do not iterate over empty slots.
+constexpr int kBandMaxE = 11;       // nodes per thread: 2 816 per SM, 416 768 per 148 SMs (645^2)
+constexpr int kBandCregE = 9;       // up to here the couplings are in registers too
+constexpr int kBandXregE = 7;       // up to here x is in registers too
+// nodes per thread of the kernel that runs ranges of n_max nodes
+inline int band_e(int n_max) { return ((n_max + kBandThreads - 1) / kBandThreads) | 1; }
+
+// u [n_max + 2 W] | M^-1 of the halo [2 W] | edges to publish [2 W] | x [n_max] (E > kBandXregE) | couplings [2][n_max + W + 1]
+// (E > kBandCregE); e: nodes per thread of the kernel that runs the range
+inline size_t band_reg_smem_bytes(int n_max, int n1, int e) {
+  return sizeof(double) * ((size_t)n_max + 6 * (size_t)n1 + (e > kBandXregE ? (size_t)n_max : 0) +
+                           (e > kBandCregE ? 2 * ((size_t)n_max + n1 + 1) : 0));
+}
+
+// What thread 0 of a block hands to the others after an exchange.
+struct BandStep {
+  double num, den, beta;   // alpha = num / den: every thread divides, beside work that needs only beta
+  int stop;                // leave the loop: converged or out of iterations
+};
+
+// The pin node: b and x0 are 0 there (cg_rhs_kernel) and M^-1 counts as 0, so
+// r, u, s and p stay 0 as long as w does; its thread sets w = 0.
+template <int E>
+__device__ __forceinline__ void cg1_band_reg_body(const BandArgs& a, const int bid, const int G) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  __shared__ BandStep step;
+  constexpr int NT = kBandThreads;
+  constexpr bool XREG = E <= kBandXregE, CREG = E <= kBandCregE;
+  const Grid3& g = a.g;
+  const int t = threadIdx.x, o0 = t * E;          // this thread's first own node
+  const int W = g.n1, NM = a.n_max;
+  const int base = (int)((long long)bid * g.ndof / G), end = (int)((long long)(bid + 1) * g.ndof / G);
+  const int nown = end - base;
+  const int mine = max(0, min(E, nown - o0));     // own nodes of this thread
+  const int pin_e = g.pin - base - o0;            // the pin among them: [0, mine), else elsewhere
+  const bool has_pin = pin_e >= 0 && pin_e < mine;
+  double* U = reinterpret_cast<double*>(smraw);   // u: [W before | range | W after]
+  double* HD = U + NM + 2 * W;                    // M^-1 of the W nodes before / after the range, 0 where unused
+  double* EV = HD + 2 * W;                        // values of the first / last W nodes that travel next
+  double* XS = EV + 2 * W;                        // !XREG: x of the range
+  double* C0 = XS + (XREG ? 0 : NM);              // !CREG: couplings to the next row [W before | range]
+  double* C1 = C0 + NM + W + 1;                   // !CREG: couplings to the next column [1 before | range]
+  FlagSlot* const edges = a.slots + (size_t)2 * G * kBandLine;   // [2 parity][G][2 side][W]
+  const int edge_set = G * 2 * W;
+
+  double r[E], w[E], sv[E], P[E], D[E], u[E], xr[XREG ? E : 1];
+  double cn[CREG ? E : 1], cs[CREG ? E : 1], ch[CREG ? E + 1 : 1];   // to the rows before / after; along the row
+  auto x_of = [&](int e) -> double& {   // of an own node, e < mine
+    if constexpr (XREG) return xr[e];
+    else return XS[o0 + e];
+  };
+  // u = M r into the shared row the neighbours' stencils read
+  auto put_u = [&](int e) {
+    u[e] = D[e] * r[e];
+    if (e < mine) U[W + o0 + e] = u[e];
+  };
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const int idx = base + o0 + e;
+    const bool in = e < mine;
+    r[e] = w[e] = sv[e] = P[e] = u[e] = 0.0;
+    if (in) x_of(e) = a.x[idx];
+    D[e] = in && e != pin_e ? a.dinv[idx] : 0.0;
+    if constexpr (CREG) {
+      cn[e] = in && idx >= W ? a.s0[idx - W] : 0.0;
+      cs[e] = in ? a.s0[idx] : 0.0;
+      if (e == 0) ch[0] = in && idx >= 1 ? a.s1[idx - 1] : 0.0;
+      ch[e + 1] = in ? a.s1[idx] : 0.0;
+    } else if (in) {
+      C0[W + o0 + e] = a.s0[idx];
+      C1[1 + o0 + e] = a.s1[idx];
+      if (o0 + e == 0) C1[0] = idx >= 1 ? a.s1[idx - 1] : 0.0;
+    }
+  }
+  // halo entry k = t + e NT: the W nodes before the range, then the W after it
+  int hoff[kBandHalo];                                  // its slot in an edge set, < 0: none
+  double hr[kBandHalo], hs[kBandHalo], hv[kBandHalo];   // its r and s, and the value that travelled last
+#pragma unroll
+  for (int e = 0; e < kBandHalo; ++e) {
+    const int k = t + e * NT, side = k >= W ? 1 : 0, kk = k - side * W;
+    const int q = side ? end + kk : base - W + kk;
+    const bool live = k < 2 * W && (side ? bid < G - 1 : bid > 0) && q >= 0 && q < g.ndof;
+    hoff[e] = live ? ((bid + (side ? 1 : -1)) * 2 + (side ^ 1)) * W + kk : -1;
+    hr[e] = hs[e] = hv[e] = 0.0;
+    if (k < 2 * W) {
+      HD[k] = live && q != g.pin ? a.dinv[q] : 0.0;
+      U[side ? nown + k : k] = live && q != g.pin && a.x_nonzero ? a.x[q] : 0.0;
+      if (!CREG && side == 0) C0[k] = live ? a.s0[q] : 0.0;
+    }
+  }
+  // S v of this thread's nodes into y: v are their own values, U holds v with
+  // the pin at 0 and the halo around the range
+  auto s_apply = [&](const double (&v)[E], double (&y)[E]) {
+    if (mine == 0) return;
+    double left = U[W + o0 - 1];
+    const double right = U[W + o0 + mine];
+    double hl;
+    if constexpr (CREG) hl = ch[0];
+    else hl = C1[o0];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      if (e < mine) {
+        const int o = o0 + e;
+        double n0, p0, p1;
+        if constexpr (CREG) {
+          n0 = cn[e]; p0 = cs[e]; p1 = ch[e + 1];
+        } else {
+          n0 = C0[o]; p0 = C0[o + W]; p1 = C1[o + 1];
+        }
+        const double next = e + 1 < E ? (e + 1 < mine ? v[e + 1 < E ? e + 1 : e] : right) : right;
+        const double d = (n0 + p0) + (hl + p1);
+        const double off = n0 * U[o] + p0 * U[o + 2 * W] + hl * left + p1 * next;
+        y[e] = d * v[e] - off;
+        left = v[e];
+        hl = p1;
+      }
+    }
+    if (has_pin) {
+#pragma unroll
+      for (int e = 0; e < E; ++e)
+        if (e == pin_e) y[e] = 0.0;
+    }
+  };
+
+  unsigned int epoch = 0;
+  // v of the range's first and last W nodes travel with the next exchange
+  // (its threads then write whole lines of slots)
+  auto publish = [&](const double (&v)[E]) {
+    if (o0 < W) {
+#pragma unroll
+      for (int e = 0; e < E; ++e)
+        if (e < mine && o0 + e < W) EV[o0 + e] = v[e];
+    }
+    const int k = o0 - (nown - W);
+    if (k + mine > 0) {
+#pragma unroll
+      for (int e = 0; e < E; ++e)
+        if (e < mine && k + e >= 0) EV[W + k + e] = v[e];
+    }
+  };
+  auto exchange = [&](const double (&red)[kBandSums], auto&& then) -> bool {
+    ++epoch;
+    const int par = (int)(epoch & 1);
+    return band_exchange(a.slots + (size_t)par * G * kBandLine, edges + (size_t)par * edge_set, a.err, G, bid, epoch,
+                         red, EV, W, hoff, hv, then);
+  };
+  // u = M r of the halo, from the r carried here
+  auto put_halo = [&](int e) {
+    const int k = t + e * NT;
+    if (k < 2 * W) U[k >= W ? nown + k : k] = HD[k] * hr[e];
+  };
+  // w = S u, the edges' w, the six inner products (all 0 on nodes beyond the range)
+  auto products = [&](double (&red)[kBandSums]) {
+    s_apply(u, w);
+    publish(w);
+#pragma unroll
+    for (int k = 0; k < kBandSums; ++k) red[k] = 0.0;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      red[0] += r[e] * u[e];
+      red[1] += w[e] * u[e];
+      red[2] += u[e] * sv[e];
+      red[3] += P[e] * w[e];
+      red[4] += P[e] * sv[e];
+      red[5] += r[e] * r[e];
+    }
+  };
+  auto finish = [&](long long it, long long applies, double rr, double bb, bool conv) {
+    if (bid == 0 && t == 0) {
+      a.st->iters = it;
+      a.st->applies = applies;
+      a.st->refinements = 0;
+      a.st->rr = rr;
+      a.st->bb = bb;
+      a.st->converged = conv ? 1 : 0;
+    }
+  };
+
+  // r0 = b - S x0 (x0 is 0 at the pin)
+  double red[kBandSums] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  if (a.x_nonzero) {
+#pragma unroll
+    for (int e = 0; e < E; ++e)
+      if (e < mine) U[W + o0 + e] = u[e] = x_of(e);
+    __syncthreads();
+    s_apply(u, w);
+  }
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    if (e < mine) {
+      const double bi = a.b[base + o0 + e];
+      r[e] = bi - w[e];   // w = S x0, or 0
+      red[0] += bi * bi;
+    }
+  }
+  publish(r);
+  // thread 0's state: (r, u), ||r||^2, ||b||^2, the limit on ||r||^2, counts
+  double gamma = 0.0, rr = 0.0, bb = 0.0, atol2 = 0.0;
+  long long it = 0;
+  const long long applies0 = a.x_nonzero ? 2 : 1;
+  bool conv = false;
+  bool ok = exchange(red, [&](const double* tot) {
+    bb = tot[0];
+    const double atol = a.tol * sqrt(bb);
+    atol2 = atol * atol;
+    step.stop = bb == 0.0;
+  });
+  if (!ok) return;
+  if (step.stop) {
+#pragma unroll
+    for (int e = 0; e < E; ++e)
+      if (e < mine) a.x[base + o0 + e] = 0.0;
+    finish(0, 0, 0.0, 0.0, true);
+    return;
+  }
+  // first pass: the edges that travelled are r; p = s = 0
+#pragma unroll
+  for (int e = 0; e < E; ++e) put_u(e);
+#pragma unroll
+  for (int e = 0; e < kBandHalo; ++e) {
+    hr[e] = hv[e];
+    put_halo(e);
+  }
+  __syncthreads();
+  products(red);
+  ok = exchange(red, [&](const double* tot) {
+    gamma = tot[0];
+    rr = tot[5];
+    conv = rr < atol2;
+    step = {gamma, tot[1], 0.0, conv || it >= a.maxiter};
+  });
+  while (ok && !step.stop) {
+    const double beta = step.beta, alpha = step.num / step.den;
+    // s, p, x, r and u = M r
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      sv[e] = __fma_rn(beta, sv[e], w[e]);
+      P[e] = u[e] + beta * P[e];
+    }
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      r[e] = __fma_rn(-alpha, sv[e], r[e]);
+      if (e < mine) x_of(e) += alpha * P[e];
+      put_u(e);
+    }
+#pragma unroll
+    for (int e = 0; e < kBandHalo; ++e) {
+      if (e * NT < 2 * W) {
+        hs[e] = __fma_rn(beta, hs[e], hv[e]);
+        hr[e] = __fma_rn(-alpha, hs[e], hr[e]);
+        put_halo(e);
+      }
+    }
+    __syncthreads();
+    products(red);
+    ok = exchange(red, [&](const double* tot) {
+      const double gnew = tot[0], be = gnew / gamma;
+      const double denom = tot[1] + be * (tot[2] + tot[3]) + be * be * tot[4];
+      gamma = gnew;
+      rr = tot[5];
+      ++it;
+      conv = rr < atol2;
+      step = {gnew, denom, be, conv || it >= a.maxiter};
+    });
+  }
+#pragma unroll
+  for (int e = 0; e < E; ++e)
+    if (e < mine) a.x[base + o0 + e] = x_of(e);
+  finish(it, applies0 + it, rr, bb, conv);
+}
+
+template <int E>
+__global__ void __launch_bounds__(kBandThreads, 1) cg1_band_kernel(BandArgs a) {
+  cg1_band_reg_body<E>(a, blockIdx.x, gridDim.x);
+}
+__global__ void __launch_bounds__(kThreads, 1) cg1_band_mixed_kernel(BandArgs a) {
+  cg1_band_mixed_body(a, blockIdx.x, gridDim.x);
 }
 
 // Many independent 2-D systems in one cooperative launch, each band-resident
-// in the shared memory of its own blocks: case c owns blocks [first[c],
-// first[c + 1]) with its own barrier counter, halo buffer and status.
+// on its own blocks: case c owns blocks [first[c], first[c + 1]) with its own
+// reduction slots (mixed: barrier counter), halo buffer and status.
 struct BandBatch {
   BandArgs c[kBatchMax];
   int first[kBatchMax + 1];
   int n;
 };
 
-template <typename T, bool MIXED>
-__global__ void __launch_bounds__(kThreads, 1) cg1_band_batch_kernel(const __grid_constant__ BandBatch b) {
+__device__ __forceinline__ int band_batch_system(const BandBatch& b) {
   int c = 0;
   while (c + 1 < b.n && (int)blockIdx.x >= b.first[c + 1]) ++c;
-  cg1_band_body<T, MIXED>(b.c[c], blockIdx.x - b.first[c], b.first[c + 1] - b.first[c]);
+  return c;
+}
+template <int E>
+__global__ void __launch_bounds__(kBandThreads, 1) cg1_band_batch_kernel(const __grid_constant__ BandBatch b) {
+  const int c = band_batch_system(b);
+  cg1_band_reg_body<E>(b.c[c], blockIdx.x - b.first[c], b.first[c + 1] - b.first[c]);
+}
+__global__ void __launch_bounds__(kThreads, 1) cg1_band_mixed_batch_kernel(const __grid_constant__ BandBatch b) {
+  const int c = band_batch_system(b);
+  cg1_band_mixed_body(b.c[c], blockIdx.x - b.first[c], b.first[c + 1] - b.first[c]);
+}
+
+// the kernel of ranges of at most n_max nodes
+void* band_kernel(int n_max, bool mixed, bool batch) {
+  if (mixed) return batch ? (void*)cg1_band_mixed_batch_kernel : (void*)cg1_band_mixed_kernel;
+  switch (band_e(n_max)) {
+    case 1: return batch ? (void*)cg1_band_batch_kernel<1> : (void*)cg1_band_kernel<1>;
+    case 3: return batch ? (void*)cg1_band_batch_kernel<3> : (void*)cg1_band_kernel<3>;
+    case 5: return batch ? (void*)cg1_band_batch_kernel<5> : (void*)cg1_band_kernel<5>;
+    case 7: return batch ? (void*)cg1_band_batch_kernel<7> : (void*)cg1_band_kernel<7>;
+    case 9: return batch ? (void*)cg1_band_batch_kernel<9> : (void*)cg1_band_kernel<9>;
+    default: return batch ? (void*)cg1_band_batch_kernel<11> : (void*)cg1_band_kernel<11>;
+  }
+}
+// shared memory of ranges of n_max nodes, 0 where they do not fit
+size_t band_smem(int n_max, int n1, bool mixed, size_t limit) {
+  if (!mixed && n_max > kBandMaxE * kBandThreads) return 0;
+  const size_t b = mixed ? band_mixed_smem_bytes(n_max, n1) : band_reg_smem_bytes(n_max, n1, band_e(n_max));
+  return b <= limit ? b : 0;
 }
 
 }  // namespace
@@ -1638,8 +2060,10 @@ struct tpf_ppe {
   int pending = 0;                     // captured CG solve: 1 status in st, 2 in cgs
   cudaStream_t cap = nullptr;          // stream the cycle is captured on (never the caller's)
   long long gm_key[6] = {};
-  double* band_pub = nullptr;     // halo rows of the band-resident PCG
+  float* band_pub = nullptr;      // halo rows of the mixed band-resident PCG
   size_t band_pub_len = 0;
+  FlagSlot* band_slots = nullptr; // sums and halo rows of the FP64 band-resident PCG
+  size_t band_slots_len = 0;
   int cg_kernel = 0;              // 0 auto, 1 global-memory persistent PCG, 2 band-resident PCG
   SolveStatus* st = nullptr;
   int coop_blocks = 0;
@@ -1863,59 +2287,74 @@ int solve_gmres(tpf_ppe* h, const double* rhs, double* p, const double* p_init, 
   return TPF_OK;
 }
 
-// band-resident PCG: applicable to 2-D systems whose largest node range
-// (one per CTA, at least one row long) fits in the opt-in shared memory of
-// one SM with 12 vectors and 6 halo rows (11 vectors and the halo in FP32
-// for the mixed mode)
+// band-resident PCG: applicable to 2-D systems whose largest node range (one
+// per CTA, at least one row long) fits on one SM: kBandMaxE nodes per thread
+// in FP64 (416 768 nodes on 148 SMs, 645^2), shared memory in the mixed mode
 struct BandPlan {
   int grid, n_max;
   size_t smem;
   bool mixed;
 };
-bool band_plan(const tpf_ppe* h, BandPlan& bp, bool mixed) {
-  if (h->cg_kernel == 1) return false;
-  const Grid3& g = h->g;
-  if (h->ndim != 2 || g.N2 != 0) return false;
-  if (2 * g.n1 > 3 * kThreads) return false;
-  const int grid = std::min(h->coop_blocks, g.ndof / g.n1);
-  if (grid < 1) return false;
-  const int n_max = (g.ndof + grid - 1) / grid;
-  const size_t smem = mixed ? band_smem_bytes<float>(n_max, g.n1) : band_smem_bytes<double>(n_max, g.n1);
+// dynamic shared memory a band kernel may use: the opt-in limit less its static scratch
+bool band_smem_limit(size_t* limit) {
   int dev = 0, optin = 0;
   cudaGetDevice(&dev);
   if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
-  // static shared memory of the kernel: the reduction scratch and GridSum's flag
-  if (smem + 4096 > (size_t)optin) return false;
-  bp.grid = grid;
-  bp.n_max = n_max;
-  bp.smem = smem;
-  bp.mixed = mixed;
+  *limit = (size_t)optin - 4096;
   return true;
 }
+// most blocks a system is spread over: one per SM, none shorter than a grid
+// row; in FP64 down to one node per thread (64^2: 2.11 us an iteration on 17
+// blocks, 2.35 on 9, 2.48 on 34; 130^2: 2.27 on 68, 2.51 on 34)
+int band_max_grid(const tpf_ppe* h, bool mixed) {
+  const Grid3& g = h->g;
+  const int most = mixed ? h->coop_blocks : std::min(tpf::sm_count(), (g.ndof + kBandThreads - 1) / kBandThreads);
+  return std::min(std::min(most, kBandMaxGrid), g.ndof / g.n1);
+}
+bool band_plan(const tpf_ppe* h, BandPlan& bp, bool mixed) {
+  if (h->cg_kernel == 1) return false;
+  const Grid3& g = h->g;
+  if (h->ndim != 2 || g.N2 != 0) return false;
+  if (g.n1 > kBandMaxW) return false;
+  const int grid = band_max_grid(h, mixed);
+  size_t limit = 0;
+  if (grid < 1 || !band_smem_limit(&limit)) return false;
+  bp.grid = grid;
+  bp.n_max = (g.ndof + grid - 1) / grid;
+  bp.smem = band_smem(bp.n_max, g.n1, mixed, limit);
+  bp.mixed = mixed;
+  return bp.smem != 0;
+}
 
-// halo buffer of a band-resident solve over `grid` blocks: [2][grid][2][3][n1]
-int ensure_band_pub(tpf_ppe* h, int grid) {
-  const size_t need = (size_t)2 * grid * 2 * 3 * h->g.n1;
-  if (h->band_pub_len < need) {
-    int st = dalloc(h, &h->band_pub, need);
-    if (st) return st;
-    h->band_pub_len = need;
+// slots of an FP64 band-resident solve over `grid` blocks: sums and edges
+size_t band_slot_count(const tpf_ppe* h, int grid) {
+  return (size_t)2 * grid * (kBandLine + 2 * (size_t)h->g.n1);
+}
+
+// exchange buffers of a band-resident solve over `grid` blocks
+int ensure_band_buffers(tpf_ppe* h, int grid, bool mixed) {
+  int st;
+  const size_t pub = (size_t)2 * grid * 2 * 3 * h->g.n1, slots = band_slot_count(h, grid);
+  if (mixed && h->band_pub_len < pub) {
+    if ((st = dalloc(h, &h->band_pub, pub))) return st;
+    h->band_pub_len = pub;
+  }
+  if (!mixed && h->band_slots_len < slots) {
+    if ((st = dalloc(h, &h->band_slots, slots))) return st;
+    h->band_slots_len = slots;
   }
   return TPF_OK;
 }
 
-int launch_band(tpf_ppe* h, const BandPlan& bp, const Cg1Args& c, cudaStream_t s) {
-  if (int st = ensure_band_pub(h, bp.grid)) return st;
-  static size_t smem_set[2] = {0, 0};
-  void* fn = bp.mixed ? (void*)cg1_band_kernel<float, true> : (void*)cg1_band_kernel<double, false>;
-  if (bp.smem > smem_set[bp.mixed]) {
-    TPF_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bp.smem));
-    smem_set[bp.mixed] = bp.smem;
-  }
-  BandArgs a{};
+// the arguments of one system's band-resident solve over `grid` blocks; the
+// slots' epochs start at 1, so their tags start at 0
+int band_args(tpf_ppe* h, int grid, int n_max, const Cg1Args& c, bool mixed, cudaStream_t s, BandArgs& a) {
+  if (int st = ensure_band_buffers(h, grid, mixed)) return st;
+  if (!mixed) TPF_CUDA_TRY(cudaMemsetAsync(h->band_slots, 0, sizeof(FlagSlot) * band_slot_count(h, grid), s));
+  a = BandArgs{};
   a.g = c.g;
   a.s0 = c.s64[0];
   a.s1 = c.s64[1];
@@ -1929,14 +2368,25 @@ int launch_band(tpf_ppe* h, const BandPlan& bp, const Cg1Args& c, cudaStream_t s
   a.tol = c.tol;
   a.replace_drop = c.replace_drop;
   a.x_nonzero = c.x_nonzero;
-  a.n_max = bp.n_max;
+  a.n_max = n_max;
   a.pub = h->band_pub;
+  a.slots = h->band_slots;
   a.part = c.part;
   a.count = c.count;
   a.err = c.err;
   a.st = c.st;
+  return TPF_OK;
+}
+
+int launch_band(tpf_ppe* h, const BandPlan& bp, const Cg1Args& c, cudaStream_t s) {
+  BandArgs a;
+  if (int st = band_args(h, bp.grid, bp.n_max, c, bp.mixed, s, a)) return st;
+  void* fn = band_kernel(bp.n_max, bp.mixed, false);
+  size_t limit = 0;
+  if (band_smem_limit(&limit))   // always the same value: other threads may launch the same kernel
+    TPF_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit));
   void* args[] = {&a};
-  TPF_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(bp.grid), dim3(kThreads), args, bp.smem, s));
+  TPF_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(bp.grid), dim3(bp.mixed ? kThreads : kBandThreads), args, bp.smem, s));
   return TPF_OK;
 }
 
@@ -2089,18 +2539,11 @@ int solve_cg_stream(tpf_ppe* h, const double* rhs, double* p, const double* p_in
   return TPF_OK;
 }
 
-int solve_cg(tpf_ppe* h, const double* rhs, double* p, const double* p_init, cudaStream_t s,
-             tpf_ppe_result* res) {
-  const Grid3& g = h->g;
-  const int n = g.ndof;
-  const Geo geo{{h->dv[0], h->dv[1], h->dv[2]}, {h->dface[0], h->dface[1], h->dface[2]}};
-  cg_rhs_kernel<<<ew_grid(h), 256, 0, s>>>(g, geo, rhs, h->b, p_init, h->x);
-  TPF_CUDA_TRY(cudaMemsetAsync(h->bar, 0, 2 * sizeof(unsigned int), s));
-  TPF_CUDA_TRY(cudaMemsetAsync(h->err, 0, sizeof(int), s));
-  TPF_CUDA_TRY(cudaMemsetAsync(h->st, 0, sizeof(SolveStatus), s));
+// the persistent kernels' view of a handle
+Cg1Args cg1_args(const tpf_ppe* h, bool x_nonzero) {
   const bool none = (h->o.precond == TPF_PRECOND_NONE);
   Cg1Args a{};
-  a.g = g;
+  a.g = h->g;
   a.v64.s0 = h->s[0]; a.v64.s1 = h->s[1]; a.v64.s2 = h->s[2];
   a.v64.dinv = none ? h->ones64 : h->dinvS;
   a.v32.s0 = h->s32[0]; a.v32.s1 = h->s32[1]; a.v32.s2 = h->s32[2];
@@ -2115,18 +2558,31 @@ int solve_cg(tpf_ppe* h, const double* rhs, double* p, const double* p_init, cud
   a.b = h->b;
   a.x = h->x;
   a.tol = h->o.tol;
-  a.x_nonzero = p_init ? 1 : 0;
+  a.maxiter = h->o.maxiter;
+  a.replace_drop = h->o.inner_tol > 0.0 ? h->o.inner_tol : 1e-3;
+  a.x_nonzero = x_nonzero ? 1 : 0;
   a.part = h->part;
   a.count = h->bar;
   a.err = h->err;
   a.st = h->st;
+  return a;
+}
+
+int solve_cg(tpf_ppe* h, const double* rhs, double* p, const double* p_init, cudaStream_t s,
+             tpf_ppe_result* res) {
+  const Grid3& g = h->g;
+  const int n = g.ndof;
+  const Geo geo{{h->dv[0], h->dv[1], h->dv[2]}, {h->dface[0], h->dface[1], h->dface[2]}};
+  cg_rhs_kernel<<<ew_grid(h), 256, 0, s>>>(g, geo, rhs, h->b, p_init, h->x);
+  TPF_CUDA_TRY(cudaMemsetAsync(h->bar, 0, 2 * sizeof(unsigned int), s));
+  TPF_CUDA_TRY(cudaMemsetAsync(h->err, 0, sizeof(int), s));
+  TPF_CUDA_TRY(cudaMemsetAsync(h->st, 0, sizeof(SolveStatus), s));
+  const Cg1Args a = cg1_args(h, p_init != nullptr);
   const bool mixed = (h->o.precision == TPF_PREC_MIXED);
   BandPlan bp;
   const bool band = band_plan(h, bp, mixed);
   if (!mixed && (h->cg_kernel == 3 || (h->cg_kernel == 0 && !band)))
     return solve_cg_stream(h, rhs, p, p_init, s, res);
-  a.maxiter = h->o.maxiter;
-  a.replace_drop = h->o.inner_tol > 0.0 ? h->o.inner_tol : 1e-3;
   if (band) {
     int st = launch_band(h, bp, a, s);
     if (st) return st;
@@ -2135,7 +2591,7 @@ int solve_cg(tpf_ppe* h, const double* rhs, double* p, const double* p_init, cud
       tpf::set_error("the band-resident PCG needs a 2-D system whose per-SM band fits in shared memory");
       return TPF_EINVAL;
     }
-    void* args[] = {&a};
+    void* args[] = {const_cast<Cg1Args*>(&a)};
     void* fn = mixed ? (void*)cg1_kernel<float, true> : (void*)cg1_kernel<double, false>;
     TPF_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(h->coop_blocks), dim3(kThreads), args, 0, s));
   }
@@ -2465,22 +2921,14 @@ namespace {
 
 // Band-resident batch: every system 2-D and the bands of all of them resident
 // at once, one block per SM.  Each system gets at least the fewest blocks
-// whose largest range fits in a block's shared memory and at most one block
+// whose largest range fits on an SM and at most one block
 // per grid row (or its single-solve grid); the blocks are shared in
 // proportion to the expected work, nodes x iterations ~ ndof^1.5, and trimmed
 // to the SM count.
 bool band_batch_plan(tpf_ppe* const* hs, int n, bool mixed, std::vector<int>& nb, std::vector<int>& nmax,
                      size_t& smem) {
-  int dev = 0, optin = 0;
-  cudaGetDevice(&dev);
-  if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
-  const size_t lim = (size_t)optin - 4096;
-  auto bytes = [&](int nm, int n1) {
-    return mixed ? band_smem_bytes<float>(nm, n1) : band_smem_bytes<double>(nm, n1);
-  };
+  size_t limit = 0;
+  if (!band_smem_limit(&limit)) return false;
   const int cap = tpf::sm_count();
   std::vector<int> lo(n), hi(n);
   double wsum = 0.0;
@@ -2488,11 +2936,12 @@ bool band_batch_plan(tpf_ppe* const* hs, int n, bool mixed, std::vector<int>& nb
   for (int c = 0; c < n; ++c) {
     const tpf_ppe* h = hs[c];
     const Grid3& g = h->g;
-    if (h->cg_kernel == 1 || h->cg_kernel == 3 || h->ndim != 2 || g.N2 != 0 || 2 * g.n1 > 3 * kThreads)
+    if (h->cg_kernel == 1 || h->cg_kernel == 3 || h->ndim != 2 || g.N2 != 0 ||
+        g.n1 > kBandMaxW)
       return false;
-    hi[c] = std::min(h->coop_blocks, g.ndof / g.n1);
+    hi[c] = band_max_grid(h, mixed);
     int k = 1;
-    while (k <= hi[c] && bytes((g.ndof + k - 1) / k, g.n1) > lim) ++k;
+    while (k <= hi[c] && !band_smem((g.ndof + k - 1) / k, g.n1, mixed, limit)) ++k;
     if (k > hi[c]) return false;
     lo[c] = k;
     sum_lo += k;
@@ -2515,8 +2964,13 @@ bool band_batch_plan(tpf_ppe* const* hs, int n, bool mixed, std::vector<int>& nb
   smem = 0;
   for (int c = 0; c < n; ++c) {
     nmax[c] = (hs[c]->g.ndof + nb[c] - 1) / nb[c];
-    smem = std::max(smem, bytes(nmax[c], hs[c]->g.n1));
+    smem = std::max(smem, band_smem(nmax[c], hs[c]->g.n1, mixed, limit));
   }
+  if (!mixed) {   // one kernel serves the batch: its layout holds for every system
+    const int e = band_e(*std::max_element(nmax.begin(), nmax.end()));
+    for (int c = 0; c < n; ++c) smem = std::max(smem, band_reg_smem_bytes(nmax[c], hs[c]->g.n1, e));
+  }
+  if (smem > limit) return false;
   return true;
 }
 
@@ -2660,41 +3114,21 @@ int launch_band_batch(tpf_ppe* const* hs, int n, const double* const* rhs, bool 
   b->first[0] = 0;
   for (int c = 0; c < n; ++c) {
     tpf_ppe* h = hs[c];
-    if (int st = ensure_band_pub(h, nb[c])) { delete b; return st; }
     const Geo geo{{h->dv[0], h->dv[1], h->dv[2]}, {h->dface[0], h->dface[1], h->dface[2]}};
     cg_rhs_kernel<<<ew_grid(h), 256, 0, s>>>(h->g, geo, rhs[c], h->b, nullptr, h->x);
     cudaMemsetAsync(h->bar, 0, 2 * sizeof(unsigned int), s);
     cudaMemsetAsync(h->err, 0, sizeof(int), s);
     cudaMemsetAsync(h->st, 0, sizeof(SolveStatus), s);
-    const bool none = (h->o.precond == TPF_PRECOND_NONE);
-    BandArgs& a = b->c[c];
-    a = BandArgs{};
-    a.g = h->g;
-    a.s0 = h->s[0];
-    a.s1 = h->s[1];
-    a.dinv = none ? h->ones64 : h->dinvS;
-    a.s0f = h->s32[0];
-    a.s1f = h->s32[1];
-    a.dinvf = none ? h->ones32 : h->dinvS32;
-    a.b = h->b;
-    a.x = h->x;
-    a.maxiter = h->o.maxiter;
-    a.tol = h->o.tol;
-    a.replace_drop = h->o.inner_tol > 0.0 ? h->o.inner_tol : 1e-3;
-    a.x_nonzero = 0;
-    a.n_max = nmax[c];
-    a.pub = h->band_pub;
-    a.part = h->part;
-    a.count = h->bar;
-    a.err = h->err;
-    a.st = h->st;
+    if (int st = band_args(h, nb[c], nmax[c], cg1_args(h, false), mixed, s, b->c[c])) { delete b; return st; }
     b->first[c + 1] = b->first[c] + nb[c];
   }
-  void* fn = mixed ? (void*)cg1_band_batch_kernel<float, true> : (void*)cg1_band_batch_kernel<double, false>;
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  void* fn = band_kernel(*std::max_element(nmax.begin(), nmax.end()), mixed, true);
+  size_t limit = smem;
+  band_smem_limit(&limit);
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit);
   if (e == cudaSuccess) {
     void* args[] = {b};
-    e = cudaLaunchCooperativeKernel(fn, dim3(b->first[n]), dim3(kThreads), args, smem, s);
+    e = cudaLaunchCooperativeKernel(fn, dim3(b->first[n]), dim3(mixed ? kThreads : kBandThreads), args, smem, s);
   }
   delete b;
   TPF_CUDA_TRY(e);
@@ -2776,31 +3210,7 @@ int tpf_ppe_solve_batched(tpf_ppe* const* hs, int n, const double* const* rhs, c
       TPF_CUDA_TRY(cudaMemsetAsync(h->bar, 0, 2 * sizeof(unsigned int), s));
       TPF_CUDA_TRY(cudaMemsetAsync(h->err, 0, sizeof(int), s));
       TPF_CUDA_TRY(cudaMemsetAsync(h->st, 0, sizeof(SolveStatus), s));
-      Cg1Args& a = b->c[c];
-      a = Cg1Args{};
-      a.g = h->g;
-      const bool none = (h->o.precond == TPF_PRECOND_NONE);
-      a.v64.s0 = h->s[0]; a.v64.s1 = h->s[1]; a.v64.s2 = h->s[2];
-      a.v64.dinv = none ? h->ones64 : h->dinvS;
-      a.v32.s0 = h->s32[0]; a.v32.s1 = h->s32[1]; a.v32.s2 = h->s32[2];
-      a.v32.dinv = none ? h->ones32 : h->dinvS32;
-      for (int k = 0; k < 2; ++k) {
-        a.v64.r[k] = h->c64[k]; a.v64.w[k] = h->c64[2 + k]; a.v64.s[k] = h->c64[4 + k];
-        a.v32.r[k] = h->c32[k]; a.v32.w[k] = h->c32[2 + k]; a.v32.s[k] = h->c32[4 + k];
-      }
-      a.v64.p = h->c64[6];
-      a.v32.p = h->c32[6];
-      a.s64[0] = h->s[0]; a.s64[1] = h->s[1]; a.s64[2] = h->s[2];
-      a.b = h->b;
-      a.x = h->x;
-      a.tol = h->o.tol;
-      a.x_nonzero = 0;
-      a.part = h->part;
-      a.count = h->bar;
-      a.err = h->err;
-      a.st = h->st;
-      a.maxiter = h->o.maxiter;
-      a.replace_drop = h->o.inner_tol > 0.0 ? h->o.inner_tol : 1e-3;
+      b->c[c] = cg1_args(h, false);
       b->first[c + 1] = b->first[c] + nb[c];
     }
     void* args[] = {b};
