@@ -31,6 +31,7 @@
 #include <cstring>
 #include <mutex>
 #include <memory>
+#include <numeric>
 #include <vector>
 
 namespace {
@@ -130,57 +131,61 @@ struct PrepArgs {
   int want_line;
 };
 
-__global__ void prep_faces_kernel(PrepArgs a) {
+// face couplings, Jacobi diagonals and line coefficients of node idx
+__device__ __forceinline__ void prep_faces_node(const PrepArgs& a, int idx) {
   const Grid3& g = a.g;
-  for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < g.ndof; idx += gridDim.x * blockDim.x) {
-    int i0, i1, i2;
-    coords3(g, idx, i0, i1, i2);
-    const int iv[3] = {i0, i1, i2};
-    const int Nv[3] = {g.N0, g.N1, g.N2};
-    const int stv[3] = {g.st0, g.n2, 1};
-    const double rho_i = a.rho[idx];
-    double dvv[3] = {a.geo.dv[0][i0], a.geo.dv[1][i1], g.N2 > 0 ? a.geo.dv[2][i2] : 1.0};
-    double diagS = 0.0, diagL = 0.0;
-    for (int ax = 0; ax < 3; ++ax) {
-      if (Nv[ax] == 0) continue;
-      double other = 1.0;
-      for (int b = 0; b < 3; ++b)
-        if (b != ax) other *= dvv[b];
-      double lower = 0.0, upper = 0.0, cf_lo = 0.0, cf_hi = 0.0;
-      if (iv[ax] > 0) {
-        double rl = a.rho[idx - stv[ax]];
-        cf_lo = 2.0 / (rl + rho_i) / a.geo.dface[ax][iv[ax] - 1];
-        lower = cf_lo / dvv[ax];
-      }
-      if (iv[ax] < Nv[ax]) {
-        double rr = a.rho[idx + stv[ax]];
-        cf_hi = 2.0 / (rho_i + rr) / a.geo.dface[ax][iv[ax]];
-        upper = cf_hi / dvv[ax];
-        double sv = cf_hi * other;
-        a.s[ax][idx] = sv;
-        a.s32[ax][idx] = (float)sv;
-      } else {
-        a.s[ax][idx] = 0.0;
-        a.s32[ax][idx] = 0.0f;
-      }
-      diagS += cf_lo * other + cf_hi * other;
-      double main = -(lower + upper);
-      diagL += main;
-      if (a.want_line) {
-        double shift = a.shift_scale / rho_i;
-        a.tlo[ax][idx] = -lower;
-        a.tdg[ax][idx] = shift - main;
-        a.tup[ax][idx] = -upper;
-      }
+  int i0, i1, i2;
+  coords3(g, idx, i0, i1, i2);
+  const int iv[3] = {i0, i1, i2};
+  const int Nv[3] = {g.N0, g.N1, g.N2};
+  const int stv[3] = {g.st0, g.n2, 1};
+  const double rho_i = a.rho[idx];
+  double dvv[3] = {a.geo.dv[0][i0], a.geo.dv[1][i1], g.N2 > 0 ? a.geo.dv[2][i2] : 1.0};
+  double diagS = 0.0, diagL = 0.0;
+  for (int ax = 0; ax < 3; ++ax) {
+    if (Nv[ax] == 0) continue;
+    double other = 1.0;
+    for (int b = 0; b < 3; ++b)
+      if (b != ax) other *= dvv[b];
+    double lower = 0.0, upper = 0.0, cf_lo = 0.0, cf_hi = 0.0;
+    if (iv[ax] > 0) {
+      double rl = a.rho[idx - stv[ax]];
+      cf_lo = 2.0 / (rl + rho_i) / a.geo.dface[ax][iv[ax] - 1];
+      lower = cf_lo / dvv[ax];
     }
-    if (idx == g.pin) {
-      diagS = 1.0;
-      diagL = 1.0;
+    if (iv[ax] < Nv[ax]) {
+      double rr = a.rho[idx + stv[ax]];
+      cf_hi = 2.0 / (rho_i + rr) / a.geo.dface[ax][iv[ax]];
+      upper = cf_hi / dvv[ax];
+      double sv = cf_hi * other;
+      a.s[ax][idx] = sv;
+      a.s32[ax][idx] = (float)sv;
+    } else {
+      a.s[ax][idx] = 0.0;
+      a.s32[ax][idx] = 0.0f;
     }
-    a.dinvS[idx] = 1.0 / diagS;
-    a.dinvS32[idx] = (float)(1.0 / diagS);
-    a.dinvL[idx] = 1.0 / (fabs(diagL) > 1e-30 ? diagL : 1.0);
+    diagS += cf_lo * other + cf_hi * other;
+    double main = -(lower + upper);
+    diagL += main;
+    if (a.want_line) {
+      double shift = a.shift_scale / rho_i;
+      a.tlo[ax][idx] = -lower;
+      a.tdg[ax][idx] = shift - main;
+      a.tup[ax][idx] = -upper;
+    }
   }
+  if (idx == g.pin) {
+    diagS = 1.0;
+    diagL = 1.0;
+  }
+  a.dinvS[idx] = 1.0 / diagS;
+  a.dinvS32[idx] = (float)(1.0 / diagS);
+  a.dinvL[idx] = 1.0 / (fabs(diagL) > 1e-30 ? diagL : 1.0);
+}
+
+__global__ void prep_faces_kernel(PrepArgs a) {
+  for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < a.g.ndof; idx += gridDim.x * blockDim.x)
+    prep_faces_node(a, idx);
 }
 
 struct LineArgs {
@@ -448,15 +453,19 @@ __global__ void apply_L_kernel(Grid3 g, Geo geo, const double* s0, const double*
 }
 
 // weighted rhs of the CG system: b = -W rhs, b[pin] = 0; x0 from p_init (pin -> 0)
+__device__ __forceinline__ void cg_rhs_node(const Grid3& g, const Geo& geo, int idx, const double* rhs, double* b,
+                                            const double* p_init, double* x) {
+  int i0, i1, i2;
+  coords3(g, idx, i0, i1, i2);
+  double W = geo.dv[0][i0] * geo.dv[1][i1] * (g.N2 > 0 ? geo.dv[2][i2] : 1.0);
+  b[idx] = (idx == g.pin) ? 0.0 : -(rhs[idx] * W);
+  x[idx] = (p_init && idx != g.pin) ? p_init[idx] : 0.0;
+}
+
 __global__ void cg_rhs_kernel(Grid3 g, Geo geo, const double* rhs, double* b, const double* p_init,
                               double* x) {
-  for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < g.ndof; idx += gridDim.x * blockDim.x) {
-    int i0, i1, i2;
-    coords3(g, idx, i0, i1, i2);
-    double W = geo.dv[0][i0] * geo.dv[1][i1] * (g.N2 > 0 ? geo.dv[2][i2] : 1.0);
-    b[idx] = (idx == g.pin) ? 0.0 : -(rhs[idx] * W);
-    x[idx] = (p_init && idx != g.pin) ? p_init[idx] : 0.0;
-  }
+  for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < g.ndof; idx += gridDim.x * blockDim.x)
+    cg_rhs_node(g, geo, idx, rhs, b, p_init, x);
 }
 
 __global__ void jacobi_L_kernel(int ndof, int pin, const double* dinvL, const double* r, double* z,
@@ -1614,6 +1623,68 @@ __global__ void __launch_bounds__(kThreads, 1) cg1_band_mixed_batch_kernel(const
   cg1_band_mixed_body(b.c[c], blockIdx.x - b.first[c], b.first[c + 1] - b.first[c]);
 }
 
+// ---- one launch before and one after a batch -------------------------------------------
+// Preparing system by system takes a launch each for the couplings, the
+// right-hand side and the result, four memsets and two copies back: at 32
+// systems ~290 launches and copies, as long as the solve itself.  The setup
+// and the finish of all systems are one launch each (system c owns the blocks
+// [first[c], first[c + 1])), and the results of all systems come back in one
+// copy.
+struct BandSetupSys {
+  PrepArgs prep;          // prep.rho NULL: the couplings are there already
+  const double* rhs;
+  double* b;
+  double* x;
+  double* p;
+  FlagSlot* slots;        // zeroed (NULL in mixed precision)
+  unsigned int n_slots;
+  unsigned int* count;
+  int* err;
+  SolveStatus* st;
+};
+struct BandSetup {
+  BandSetupSys c[kBatchMax];
+  int first[kBatchMax + 1];
+  int n;
+};
+struct BandOutcome {
+  SolveStatus st;
+  int err, pad;
+};
+
+__device__ __forceinline__ int band_setup_system(const BandSetup& b) {
+  int c = 0;
+  while (c + 1 < b.n && (int)blockIdx.x >= b.first[c + 1]) ++c;
+  return c;
+}
+
+__global__ void __launch_bounds__(256) band_setup_kernel(const __grid_constant__ BandSetup b) {
+  const int c = band_setup_system(b);
+  const BandSetupSys& y = b.c[c];
+  const int gt = (blockIdx.x - b.first[c]) * blockDim.x + threadIdx.x, nt = (b.first[c + 1] - b.first[c]) * blockDim.x;
+  const Grid3& g = y.prep.g;
+  for (int idx = gt; idx < g.ndof; idx += nt) {
+    if (y.prep.rho) prep_faces_node(y.prep, idx);
+    cg_rhs_node(g, y.prep.geo, idx, y.rhs, y.b, nullptr, y.x);
+  }
+  for (unsigned int k = gt; k < y.n_slots; k += nt) y.slots[k] = {0, 0};
+  if (gt == 0) {
+    *y.count = 0u;
+    *y.err = 0;
+    *y.st = SolveStatus{};
+  }
+}
+
+// p = x with p[pin] = 0, and every system's status into out[c]
+__global__ void __launch_bounds__(256) band_finish_kernel(const __grid_constant__ BandSetup b, BandOutcome* out) {
+  const int c = band_setup_system(b);
+  const BandSetupSys& y = b.c[c];
+  const int gt = (blockIdx.x - b.first[c]) * blockDim.x + threadIdx.x, nt = (b.first[c + 1] - b.first[c]) * blockDim.x;
+  const Grid3& g = y.prep.g;
+  for (int idx = gt; idx < g.ndof; idx += nt) y.p[idx] = idx == g.pin ? 0.0 : y.x[idx];
+  if (gt == 0) out[c] = {*y.st, *y.err, 0};
+}
+
 // the kernel of ranges of at most n_max nodes
 void* band_kernel(int n_max, bool mixed, bool batch) {
   if (mixed) return batch ? (void*)cg1_band_mixed_batch_kernel : (void*)cg1_band_mixed_kernel;
@@ -2056,6 +2127,8 @@ struct tpf_ppe {
   cudaGraphExec_t cg_exec = nullptr;   // a chunk of streaming-PCG iterations, captured
   long long cg_key[6] = {};
   void* cgs = nullptr;                 // streaming-PCG device scalars (CgScal)
+  BandOutcome* batch_out = nullptr;    // per system: status of a band-resident batch
+  int batch_out_len = 0;
   int* batch_pending = nullptr;        // systems still iterating in a batched streaming solve
   int pending = 0;                     // captured CG solve: 1 status in st, 2 in cgs
   cudaStream_t cap = nullptr;          // stream the cycle is captured on (never the caller's)
@@ -2349,11 +2422,10 @@ int ensure_band_buffers(tpf_ppe* h, int grid, bool mixed) {
   return TPF_OK;
 }
 
-// the arguments of one system's band-resident solve over `grid` blocks; the
-// slots' epochs start at 1, so their tags start at 0
-int band_args(tpf_ppe* h, int grid, int n_max, const Cg1Args& c, bool mixed, cudaStream_t s, BandArgs& a) {
+// the arguments of one system's band-resident solve over `grid` blocks; its
+// slots' tags start at 0 (the epochs at 1)
+int band_args(tpf_ppe* h, int grid, int n_max, const Cg1Args& c, bool mixed, BandArgs& a) {
   if (int st = ensure_band_buffers(h, grid, mixed)) return st;
-  if (!mixed) TPF_CUDA_TRY(cudaMemsetAsync(h->band_slots, 0, sizeof(FlagSlot) * band_slot_count(h, grid), s));
   a = BandArgs{};
   a.g = c.g;
   a.s0 = c.s64[0];
@@ -2380,7 +2452,9 @@ int band_args(tpf_ppe* h, int grid, int n_max, const Cg1Args& c, bool mixed, cud
 
 int launch_band(tpf_ppe* h, const BandPlan& bp, const Cg1Args& c, cudaStream_t s) {
   BandArgs a;
-  if (int st = band_args(h, bp.grid, bp.n_max, c, bp.mixed, s, a)) return st;
+  if (int st = band_args(h, bp.grid, bp.n_max, c, bp.mixed, a)) return st;
+  if (!bp.mixed)
+    TPF_CUDA_TRY(cudaMemsetAsync(h->band_slots, 0, sizeof(FlagSlot) * band_slot_count(h, bp.grid), s));
   void* fn = band_kernel(bp.n_max, bp.mixed, false);
   size_t limit = 0;
   if (band_smem_limit(&limit))   // always the same value: other threads may launch the same kernel
@@ -2537,6 +2611,28 @@ int solve_cg_stream(tpf_ppe* h, const double* rhs, double* p, const double* p_in
     return TPF_ENOCONV;
   }
   return TPF_OK;
+}
+
+PrepArgs prep_args(const tpf_ppe* h, const double* rho) {
+  PrepArgs a{};
+  a.g = h->g;
+  a.geo = Geo{{h->dv[0], h->dv[1], h->dv[2]}, {h->dface[0], h->dface[1], h->dface[2]}};
+  a.rho = rho;
+  for (int ax = 0; ax < 3; ++ax) {
+    a.s[ax] = (ax < h->ndim) ? h->s[ax] : nullptr;
+    a.s32[ax] = (ax < h->ndim) ? h->s32[ax] : nullptr;
+    a.tlo[ax] = (ax < h->ndim) ? h->tlo[ax] : nullptr;
+    a.tdg[ax] = (ax < h->ndim) ? h->tden[ax] : nullptr;
+    a.tup[ax] = (ax < h->ndim) ? h->tcp[ax] : nullptr;
+  }
+  a.dinvS = h->dinvS;
+  a.dinvS32 = h->dinvS32;
+  a.dinvL = h->dinvL;
+  a.shift_scale = 2.0 / (h->o.c_tau * h->h_min * h->h_min);
+  a.ndim = h->ndim;
+  // the shifted line systems and their Thomas factors only for the line preconditioner
+  a.want_line = (h->o.precond == TPF_PRECOND_LINE || h->o.precond == TPF_PRECOND_LINE_PCR) ? 1 : 0;
+  return a;
 }
 
 // the persistent kernels' view of a handle
@@ -2810,25 +2906,8 @@ int tpf_ppe_set_options(tpf_ppe* h, const tpf_ppe_options* o) {
 int tpf_ppe_prepare(tpf_ppe* h, const double* rho, void* stream) {
   TPF_CHECK_ARG(h && rho, "NULL argument");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  PrepArgs a{};
-  a.g = h->g;
-  a.geo = Geo{{h->dv[0], h->dv[1], h->dv[2]}, {h->dface[0], h->dface[1], h->dface[2]}};
-  a.rho = rho;
-  for (int ax = 0; ax < 3; ++ax) {
-    a.s[ax] = (ax < h->ndim) ? h->s[ax] : nullptr;
-    a.s32[ax] = (ax < h->ndim) ? h->s32[ax] : nullptr;
-    a.tlo[ax] = (ax < h->ndim) ? h->tlo[ax] : nullptr;
-    a.tdg[ax] = (ax < h->ndim) ? h->tden[ax] : nullptr;
-    a.tup[ax] = (ax < h->ndim) ? h->tcp[ax] : nullptr;
-  }
-  a.dinvS = h->dinvS;
-  a.dinvS32 = h->dinvS32;
-  a.dinvL = h->dinvL;
-  a.shift_scale = 2.0 / (h->o.c_tau * h->h_min * h->h_min);
-  a.ndim = h->ndim;
-  // the shifted line systems and their Thomas factors only for the line preconditioner
-  const bool line = (h->o.precond == TPF_PRECOND_LINE || h->o.precond == TPF_PRECOND_LINE_PCR);
-  a.want_line = line ? 1 : 0;
+  const PrepArgs a = prep_args(h, rho);
+  const bool line = a.want_line != 0;
   prep_faces_kernel<<<h->ew_blocks, 256, 0, s>>>(a);
   TPF_CUDA_TRY(cudaGetLastError());
   // Thomas factors for the exact line solve; truncated PCR works on the raw coefficients
@@ -2921,10 +3000,16 @@ namespace {
 
 // Band-resident batch: every system 2-D and the bands of all of them resident
 // at once, one block per SM.  Each system gets at least the fewest blocks
-// whose largest range fits on an SM and at most one block
-// per grid row (or its single-solve grid); the blocks are shared in
-// proportion to the expected work, nodes x iterations ~ ndof^1.5, and trimmed
-// to the SM count.
+// whose largest range fits and at most one block per grid row (or its
+// single-solve grid).
+// FP64: one kernel runs all systems, so the blocks start from the smallest
+// nodes per thread E with which every system fits, and the rest go one by one
+// to the system that would finish last: iterations ~ sqrt(nodes), each
+// ~2.1 us + 0.9 us per 1 000 nodes of its largest range (64^2 and 512^2
+// measured).  Shares by nodes^1.5 alone left the smallest systems on one block
+// and the batch on E = 11: 32 systems of 48..96 took 2.32 ms in the kernel.
+// Mixed precision: shares in proportion to nodes x iterations ~ ndof^1.5,
+// trimmed to the SM count.
 bool band_batch_plan(tpf_ppe* const* hs, int n, bool mixed, std::vector<int>& nb, std::vector<int>& nmax,
                      size_t& smem) {
   size_t limit = 0;
@@ -2932,7 +3017,6 @@ bool band_batch_plan(tpf_ppe* const* hs, int n, bool mixed, std::vector<int>& nb
   const int cap = tpf::sm_count();
   std::vector<int> lo(n), hi(n);
   double wsum = 0.0;
-  int sum_lo = 0;
   for (int c = 0; c < n; ++c) {
     const tpf_ppe* h = hs[c];
     const Grid3& g = h->g;
@@ -2944,11 +3028,35 @@ bool band_batch_plan(tpf_ppe* const* hs, int n, bool mixed, std::vector<int>& nb
     while (k <= hi[c] && !band_smem((g.ndof + k - 1) / k, g.n1, mixed, limit)) ++k;
     if (k > hi[c]) return false;
     lo[c] = k;
-    sum_lo += k;
     wsum += std::pow((double)g.ndof, 1.5);
   }
-  if (sum_lo > cap) return false;
+  if (std::accumulate(lo.begin(), lo.end(), 0) > cap) return false;
   int used = 0;
+  if (!mixed) {
+    for (int e = 1; e <= kBandMaxE; e += 2) {
+      used = 0;
+      for (int c = 0; c < n; ++c) {
+        nb[c] = std::max(lo[c], std::min(hi[c], (hs[c]->g.ndof + e * kBandThreads - 1) / (e * kBandThreads)));
+        used += nb[c];
+      }
+      if (used <= cap) break;
+    }
+    if (used > cap) {   // a system short of blocks for its share of E (its rows are long)
+      nb = lo;
+      used = std::accumulate(lo.begin(), lo.end(), 0);
+    }
+    auto work = [&](int c) {
+      const double nodes = hs[c]->g.ndof;
+      return std::sqrt(nodes) * (2300.0 + nodes / nb[c]);
+    };
+    for (; used < cap; ++used) {
+      int m = -1;
+      for (int c = 0; c < n; ++c)
+        if (nb[c] < hi[c] && (m < 0 || work(c) > work(m))) m = c;
+      if (m < 0) break;
+      ++nb[m];
+    }
+  } else {
   for (int c = 0; c < n; ++c) {
     const int share = (int)((double)cap * std::pow((double)hs[c]->g.ndof, 1.5) / wsum);
     nb[c] = std::max(lo[c], std::min(hi[c], share));
@@ -2960,6 +3068,7 @@ bool band_batch_plan(tpf_ppe* const* hs, int n, bool mixed, std::vector<int>& nb
       if (nb[c] > lo[c] && (m < 0 || nb[c] > nb[m])) m = c;
     --nb[m];
     --used;
+  }
   }
   smem = 0;
   for (int c = 0; c < n; ++c) {
@@ -3107,31 +3216,54 @@ int solve_cgs_batch(tpf_ppe* const* hs, int n, const double* const* rhs, double*
   return status;
 }
 
-int launch_band_batch(tpf_ppe* const* hs, int n, const double* const* rhs, bool mixed, const std::vector<int>& nb,
-                      const std::vector<int>& nmax, size_t smem, cudaStream_t s) {
-  auto* b = new BandBatch();
-  b->n = n;
-  b->first[0] = 0;
+// One band-resident launch for the whole batch, with the setup before it and
+// the results after it in one launch each; results[c] and the batch status.
+int solve_band_batch(tpf_ppe* const* hs, int n, const double* const* rhs, const double* const* rho,
+                     double* const* p, bool mixed, const std::vector<int>& nb, const std::vector<int>& nmax,
+                     size_t smem, cudaStream_t s, BandOutcome* out) {
+  std::unique_ptr<BandBatch> b(new BandBatch());
+  std::unique_ptr<BandSetup> u(new BandSetup());
+  b->n = u->n = n;
+  b->first[0] = u->first[0] = 0;
+  int st;
   for (int c = 0; c < n; ++c) {
     tpf_ppe* h = hs[c];
-    const Geo geo{{h->dv[0], h->dv[1], h->dv[2]}, {h->dface[0], h->dface[1], h->dface[2]}};
-    cg_rhs_kernel<<<ew_grid(h), 256, 0, s>>>(h->g, geo, rhs[c], h->b, nullptr, h->x);
-    cudaMemsetAsync(h->bar, 0, 2 * sizeof(unsigned int), s);
-    cudaMemsetAsync(h->err, 0, sizeof(int), s);
-    cudaMemsetAsync(h->st, 0, sizeof(SolveStatus), s);
-    if (int st = band_args(h, nb[c], nmax[c], cg1_args(h, false), mixed, s, b->c[c])) { delete b; return st; }
+    if ((st = band_args(h, nb[c], nmax[c], cg1_args(h, false), mixed, b->c[c]))) return st;
+    BandSetupSys& y = u->c[c];
+    y.prep = prep_args(h, rho ? rho[c] : nullptr);
+    y.rhs = rhs[c];
+    y.b = h->b;
+    y.x = h->x;
+    y.p = p[c];
+    y.slots = mixed ? nullptr : h->band_slots;
+    y.n_slots = mixed ? 0u : (unsigned int)band_slot_count(h, nb[c]);
+    y.count = h->bar;
+    y.err = h->err;
+    y.st = h->st;
     b->first[c + 1] = b->first[c] + nb[c];
+    u->first[c + 1] = u->first[c] + std::min(h->ew_blocks, std::max(1, (h->g.ndof + 511) / 512));
+    if (y.prep.rho) {
+      h->line_ready = 0;
+      h->prepared = true;
+    }
+  }
+  tpf_ppe* h0 = hs[0];
+  if (h0->batch_out_len < n) {
+    if ((st = dalloc(h0, &h0->batch_out, (size_t)n))) return st;
+    h0->batch_out_len = n;
   }
   void* fn = band_kernel(*std::max_element(nmax.begin(), nmax.end()), mixed, true);
   size_t limit = smem;
   band_smem_limit(&limit);
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit);
-  if (e == cudaSuccess) {
-    void* args[] = {b};
-    e = cudaLaunchCooperativeKernel(fn, dim3(b->first[n]), dim3(mixed ? kThreads : kBandThreads), args, smem, s);
-  }
-  delete b;
-  TPF_CUDA_TRY(e);
+  TPF_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit));
+  band_setup_kernel<<<u->first[n], 256, 0, s>>>(*u);
+  void* args[] = {b.get()};
+  TPF_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(b->first[n]), dim3(mixed ? kThreads : kBandThreads), args, smem,
+                                           s));
+  band_finish_kernel<<<u->first[n], 256, 0, s>>>(*u, h0->batch_out);
+  TPF_CUDA_TRY(cudaGetLastError());
+  TPF_CUDA_TRY(cudaMemcpyAsync(out, h0->batch_out, sizeof(BandOutcome) * (size_t)n, cudaMemcpyDeviceToHost, s));
+  TPF_CUDA_TRY(cudaStreamSynchronize(s));
   return TPF_OK;
 }
 
@@ -3151,9 +3283,14 @@ int tpf_ppe_solve_batched(tpf_ppe* const* hs, int n, const double* const* rhs, c
     TPF_CHECK_ARG(h && rhs[c] && p[c], "NULL handle or array for system %d", c);
     TPF_CHECK_ARG(h->o.method == TPF_PPE_CG, "batched solves run the CG route (system %d)", c);
     TPF_CHECK_ARG((h->o.precision == TPF_PREC_MIXED) == mixed, "all systems of a batch share one precision");
-    if (rho && rho[c] && (st = tpf_ppe_prepare(h, rho[c], stream))) return st;
-    TPF_CHECK_ARG(h->prepared, "operator coefficients of system %d are not initialised", c);
+    TPF_CHECK_ARG(h->prepared || (rho && rho[c]), "operator coefficients of system %d are not initialised", c);
   }
+  auto prepare = [&]() -> int {   // the couplings, one system after the other
+    for (int c = 0; c < n; ++c)
+      if (rho && rho[c])
+        if (int e = tpf_ppe_prepare(hs[c], rho[c], stream)) return e;
+    return TPF_OK;
+  };
   // the band-resident batch where every band fits at once, else the
   // all-global persistent body
   std::vector<int> bnb(n), bnmax(n);
@@ -3165,11 +3302,15 @@ int tpf_ppe_solve_batched(tpf_ppe* const* hs, int n, const double* const* rhs, c
     force_global = force_global || hs[c]->cg_kernel == 1;
     force_stream = force_stream || hs[c]->cg_kernel == 3;
   }
-  TPF_CHECK_ARG(!(force_stream && (force_band || force_global)), "conflicting CG kernel choices in one batch");
-  TPF_CHECK_ARG(!(force_stream && mixed), "the batched streaming PCG runs FP64 systems");
+  std::vector<BandOutcome> out(n);
+  const bool refused = force_stream && (force_band || force_global || mixed);
+  const bool band = !force_stream && band_batch_plan(hs, n, mixed, bnb, bnmax, bsmem);
+  if (!band && (st = prepare())) return st;   // the band-resident batch prepares in its own setup
+  TPF_CHECK_ARG(!(refused && !mixed), "conflicting CG kernel choices in one batch");
+  TPF_CHECK_ARG(!refused, "the batched streaming PCG runs FP64 systems");
   if (force_stream) return solve_cgs_batch(hs, n, rhs, p, s, results);
-  if (band_batch_plan(hs, n, mixed, bnb, bnmax, bsmem)) {
-    if ((st = launch_band_batch(hs, n, rhs, mixed, bnb, bnmax, bsmem, s))) return st;
+  if (band) {
+    if ((st = solve_band_batch(hs, n, rhs, rho, p, mixed, bnb, bnmax, bsmem, s, out.data()))) return st;
   } else if (force_band) {
     tpf::set_error("the band-resident batch needs 2-D systems whose bands all fit in shared memory at once");
     return TPF_EINVAL;
@@ -3217,29 +3358,27 @@ int tpf_ppe_solve_batched(tpf_ppe* const* hs, int n, const double* const* rhs, c
     cudaError_t e = cudaLaunchCooperativeKernel(fn, dim3(b->first[n]), dim3(kThreads), args, 0, s);
     delete b;
     TPF_CUDA_TRY(e);
+    for (int c = 0; c < n; ++c) {
+      tpf_ppe* h = hs[c];
+      copy_pin0_kernel<<<ew_grid(h), 256, 0, s>>>(h->g.ndof, h->g.pin, h->x, p[c]);
+      TPF_CUDA_TRY(cudaMemcpyAsync(&out[c].st, h->st, sizeof(SolveStatus), cudaMemcpyDeviceToHost, s));
+      TPF_CUDA_TRY(cudaMemcpyAsync(&out[c].err, h->err, sizeof(int), cudaMemcpyDeviceToHost, s));
+    }
+    TPF_CUDA_TRY(cudaStreamSynchronize(s));
   }
-  std::vector<SolveStatus> hst(n);
-  std::vector<int> herr(n);
-  for (int c = 0; c < n; ++c) {
-    tpf_ppe* h = hs[c];
-    copy_pin0_kernel<<<ew_grid(h), 256, 0, s>>>(h->g.ndof, h->g.pin, h->x, p[c]);
-    TPF_CUDA_TRY(cudaMemcpyAsync(&hst[c], h->st, sizeof(SolveStatus), cudaMemcpyDeviceToHost, s));
-    TPF_CUDA_TRY(cudaMemcpyAsync(&herr[c], h->err, sizeof(int), cudaMemcpyDeviceToHost, s));
-  }
-  TPF_CUDA_TRY(cudaStreamSynchronize(s));
   int status = TPF_OK;
   for (int c = 0; c < n; ++c) {
     tpf_ppe_result r{};
-    r.iterations = hst[c].iters;
-    r.applies = hst[c].applies;
-    r.refinements = hst[c].refinements;
-    r.rel_residual = hst[c].bb > 0.0 ? std::sqrt(hst[c].rr / hst[c].bb) : 0.0;
-    r.info = hst[c].converged ? 0 : (int)std::min<long long>(hs[c]->o.maxiter, 0x7fffffff);
+    r.iterations = out[c].st.iters;
+    r.applies = out[c].st.applies;
+    r.refinements = out[c].st.refinements;
+    r.rel_residual = out[c].st.bb > 0.0 ? std::sqrt(out[c].st.rr / out[c].st.bb) : 0.0;
+    r.info = out[c].st.converged ? 0 : (int)std::min<long long>(hs[c]->o.maxiter, 0x7fffffff);
     if (results) results[c] = r;
-    if (herr[c]) {
+    if (out[c].err) {
       tpf::set_error("PCG barrier of batched system %d timed out; the solve was aborted", c);
       status = TPF_EABORT;
-    } else if (!hst[c].converged && status == TPF_OK) {
+    } else if (!out[c].st.converged && status == TPF_OK) {
       tpf::set_error("batched PCG system %d did not converge (info=%d)", c, r.info);
       status = TPF_ENOCONV;
     }
