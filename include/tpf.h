@@ -60,8 +60,7 @@ const char* tpf_last_error(void);
  * shape.  mode 1 (default) tunes; 0 switches tuning off and forgets the
  * choices (the heuristic shapes are then used); 2 + k makes every tuned
  * kernel take its candidate k (clamped to its last one) without timing, to
- * check that every shape gives the same bits.  The CCD plans carry their own
- * autotuner (tpf_ccd_plan_set_autotune). */
+ * check that every shape gives the same bits. */
 int tpf_set_launch_autotune(int mode);
 /* Number of signatures tuned so far in this process. */
 int tpf_launch_autotune_entries(void);
@@ -83,14 +82,9 @@ int tpf_ccd_plan_create(tpf_ccd_plan** plan, int64_t n_pts, double h, int bc,
                         int dtype);
 int tpf_ccd_plan_destroy(tpf_ccd_plan* plan);
 
-/* Launch-shape autotuning of the line kernels (default on; no counterpart
- * in the reference): the first tpf_ccd_apply of each (line count, axis kind,
- * boundary, outputs, dtype) combination times a few launch shapes on the
- * caller's stream and keeps the fastest -- warps per block and tile ring depth
- * of the lane-per-line kernel (3-D grids), lines per block and tile buffers of
- * the warp kernel (2-D grids) -- results are identical for every shape.  That first call synchronizes the stream; it is skipped while the
- * stream is being captured.  enable = 0 switches tuning off and forgets the
- * choices. */
+/* Kept for callers of earlier versions, without effect: the launch shapes of
+ * the line kernels follow from the sizes, and the results do not depend on
+ * them. */
 int tpf_ccd_plan_set_autotune(tpf_ccd_plan* plan, int enable);
 
 /* Metric of a non-uniform axis (host arrays of n_pts doubles: J = dxi/dx and

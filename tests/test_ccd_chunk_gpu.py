@@ -1,0 +1,104 @@
+"""The chunk-per-thread CCD kernels at the edges of their chunks, windows and tiles."""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+from oracle import ccd as occd  # noqa: E402
+
+# nodes of a line: shorter than a chunk of 16 rows, just around one, two and five chunks (the window is four) and
+# the 48 head rows; a multiple of 4 (padded pitch); the most rows of 8, 4 and 2 lines per block; beyond them
+LENGTHS = [6, 7, 17, 18, 19, 33, 34, 35, 49, 50, 51, 66, 81, 82, 84, 256, 1026, 1027, 2050, 2051, 4098, 4099]
+
+
+def _tol(f, h, order):
+    """1e-12 of the result plus the round-off of the wall closure's own sum,
+    8 eps max|f| sum|c| (c_I: 10.7 / h, c_II: 640 / 12 h^2)."""
+    c = 10.7 / h if order == 1 else 640.0 / (12.0 * h * h)
+    return 8 * np.finfo(np.float64).eps * np.abs(f).max() * c
+
+
+@pytest.mark.parametrize("n", LENGTHS)
+@pytest.mark.parametrize("bc", ["wall", "periodic"])
+@pytest.mark.parametrize("axis", [0, 1])
+def test_line_lengths_and_ragged_tiles(cuda_device, n, bc, axis):
+    """37 lines (no multiple of a tile) of every length, as rows and as
+    columns, against the oracle's dense solve; a view that starts off 16 bytes
+    gives the same bits."""
+    import torch
+    from twophaseflow_b200 import CCDSolver, UniformGrid
+    shape = (n, 37) if axis == 0 else (37, n)
+    N = tuple(s - 1 for s in shape)
+    f = np.random.default_rng(n).standard_normal(shape)
+    if bc == "periodic":
+        f[-1, :] = f[0, :]
+        f[:, -1] = f[:, 0]
+    ccd = CCDSolver(UniformGrid(N), None, bc_type=bc)
+    store = torch.zeros(f.size + 1, dtype=torch.float64, device=cuda_device)
+    store[1:] = torch.from_numpy(f.ravel()).to(cuda_device)
+    d = ccd.differentiate(torch.from_numpy(f).to(cuda_device), axis)
+    u = ccd.differentiate(store[1:].view(shape), axis)
+    h = 1.0 / N[axis]
+    # the dense 2 n x 2 n solve of the longest lines takes minutes: their middle is compared with the solve of a
+    # window of 801 nodes, whose ends are 300 rows away (0.455^300 of them is left)
+    for k in range(2):
+        assert torch.equal(d[k], u[k])
+        got = np.moveaxis(d[k].cpu().numpy(), axis, 0)
+        line = np.moveaxis(f, axis, 0)
+        if n <= 1027:
+            ref = np.moveaxis(occd.differentiate(f, axis, h, bc=bc)[k], axis, 0)
+            err = np.abs(got - ref).max()
+            tol = 1e-12 * np.abs(ref).max() + (_tol(f, h, k + 1) if bc == "wall" else 0.0)
+            assert err <= tol, (k, err, tol)
+            continue
+        for a in (0, n // 2 - 400, n - 801):
+            w = occd.differentiate(np.ascontiguousarray(line[a:a + 801]), 0, h, bc="wall")[k]
+            lo = 0 if a == 0 and bc == "wall" else 300
+            hi = 801 if a == n - 801 and bc == "wall" else 501
+            err = np.abs(got[a + lo:a + hi] - w[lo:hi]).max()
+            assert err <= 1e-12 * np.abs(w).max() + _tol(f, h, k + 1), (k, a, err)
+
+
+@pytest.mark.parametrize("shape,axis", [((300, 200, 160), 0), ((160, 300, 200), 1), ((257, 129, 130), 0),
+                                        ((100, 90, 200), 2), ((64, 600, 100), 1)])
+@pytest.mark.parametrize("dtype", ["f64", "f32"])
+def test_many_lines_match_the_single_line_solve(cuda_device, shape, axis, dtype):
+    """The tile width and the staged copies do not enter a line's arithmetic:
+    each line of a large field has the bits of its own one-line solve."""
+    import torch
+    from twophaseflow_b200 import CCDSolver, UniformGrid
+    dt = torch.float64 if dtype == "f64" else torch.float32
+    f = torch.randn(shape, device=cuda_device, dtype=dt, generator=torch.Generator(device="cuda").manual_seed(3))
+    N = tuple(s - 1 for s in shape)
+    d = CCDSolver(UniformGrid(N), None, bc_type="wall", dtype=dt).differentiate(f, axis)
+    n = shape[axis]
+    one = CCDSolver(UniformGrid((n - 1, 6), (1.0, 1.0)), None, bc_type="wall", dtype=dt)
+    lines = [t.movedim(axis, 0).reshape(n, -1) for t in (f, *d)]
+    m = lines[0].shape[1]
+    for c in (0, 1, 15, 16, 31, 32, m // 2 - 3, m - 7):
+        cols = slice(c, c + 7)
+        e = one.differentiate(lines[0][:, cols].contiguous(), 0)
+        for k in range(2):
+            assert torch.equal(e[k], lines[1 + k][:, cols]), (c, k)
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("bc", ["wall", "periodic"])
+@pytest.mark.parametrize("axis", [0, 1])
+def test_one_bad_value_reaches_its_whole_line(cuda_device, bad, bc, axis):
+    """The recurrences carry a value that is not finite from end to end of its
+    line, however far the chunks' windows reach, and to no other line."""
+    import torch
+    from twophaseflow_b200 import CCDSolver, UniformGrid
+    f = torch.randn((400, 400), device=cuda_device, dtype=torch.float64)
+    if bc == "periodic":
+        f[-1], f[:, -1] = f[0].clone(), f[:, 0].clone()
+        f[-1, -1] = f[0, 0]
+    f[200, 200] = bad
+    d = CCDSolver(UniformGrid((399, 399)), None, bc_type=bc).differentiate(f, axis)
+    for t in d:
+        finite = torch.isfinite(t.movedim(axis, 0))
+        assert not bool(finite[:, 200].any())
+        finite[:, 200] = True
+        assert bool(finite.all())

@@ -10,7 +10,9 @@
 //
 // Algorithm (this file's own design, not the reference's dense LU):
 // the block matrix is the same for every line, so its 2x2 block-LU factors
-// (block_tridiag.py:67-104) are computed once on the host.  Every line is cut
+// (block_tridiag.py:67-104) are computed once on the host.  Lines of up to
+// 4 096 rows are solved by the chunk kernels of ccd_chunk.cuh; the kernel below
+// takes longer ones.  Every line is cut
 // into P chunks of C rows; each chunk runs the forward/backward block-Thomas
 // sweeps locally, and the exact coupling between chunks is restored by a short
 // scan over the chunk carries (the sweeps are affine first-order recurrences
@@ -29,11 +31,7 @@
 #include <vector>
 #include <array>
 #include <algorithm>
-#include <map>
-
-struct LaneShape_ {
-  int warps, nbuf, max_bps;
-};
+#include <type_traits>
 
 namespace {
 
@@ -57,6 +55,21 @@ inline M2 eye() { return {1.0, 0.0, 0.0, 1.0}; }
 inline double maxabs(const M2& a) {
   return std::max(std::max(std::fabs(a[0]), std::fabs(a[1])), std::max(std::fabs(a[2]), std::fabs(a[3])));
 }
+
+// ---- chunk kernels (ccd_chunk.cuh) ----
+constexpr int kChunkWindow = 4;
+constexpr int kChunkHead = 48;   // 0.455^48 = 4e-17
+constexpr int kChunkR = 16;
+
+// constants of a plan for chunks of R rows, in the compute type
+template <typename T, int R>
+struct ChunkConst {
+  T A[4], AR[4], B[4], BR[4];     // A (scaled) and B, and their R-th powers
+  T P[4], Z[4];                   // P (scaled), P_last P^-1
+  T Gf[4], Gb[4], AL[4], BL[4];   // periodic: ring closures, A and B to the power of the last chunk's rows
+  T cl[4], cr[4];                 // closure -> first right-hand side (scaled) / last solution
+  double Ml[4], Mr[4], cIl[4], cIr[4], cII[6];   // wall closures
+};
 
 // Table layout (doubles).  C = chunk length, H0 = rows [0, H0) of the wall
 // "head" that carry per-row factors (the block-LU factors only reach the
@@ -83,14 +96,11 @@ struct tpf_ccd_plan {
   float* d_tabf = nullptr;   // float copy (interior factors for F32)
   double* d_J = nullptr;     // metric J, dJ (n_pts each)
   bool has_metric = false;
-  // lane-per-line kernel table (factors, ring closures, head rows)
-  double* d_ltab = nullptr;
-  float* d_ltabf = nullptr;
-  int ltab_total = 0;
-  std::vector<double> ltab_host;
-  // lane-kernel launch shapes picked by the autotuner, per call signature
-  mutable std::map<uint64_t, LaneShape_> lane_tuned;
-  bool autotune = true;
+  // constants of the chunk kernels, and their wall tables G [kChunkHead + kChunkR][4]
+  ChunkConst<double, kChunkR> c64;
+  ChunkConst<float, kChunkR> c32;
+  double* d_g64 = nullptr;
+  float* d_g32 = nullptr;
   // FP32 per-row block-LU factors of the folded wall system (Lf, P, H per
   // row) for the iterative-refinement correction solves, built on first use
   mutable float* d_rfac = nullptr;
@@ -172,26 +182,6 @@ __device__ __forceinline__ void cp_async(void* smem, const void* gmem, bool vali
   int src = valid ? BYTES : 0;   // src-size 0 -> zero fill
   asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(sa), "l"(gmem), "n"(BYTES), "r"(src)
                : "memory");
-}
-// cp.async with an L2 eviction-priority policy (createpolicy), for staging
-// copies whose lines are re-read later (evict_last) or read for the last
-// time (evict_first)
-template <int BYTES>
-__device__ __forceinline__ void cp_async_pol(void* smem, const void* gmem, uint64_t pol) {
-  unsigned int sa = (unsigned int)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global.L2::cache_hint [%0], [%1], %2, %2, %3;\n" ::"r"(sa), "l"(gmem), "n"(BYTES),
-               "l"(pol)
-               : "memory");
-}
-__device__ __forceinline__ uint64_t pol_evict_last() {
-  uint64_t p;
-  asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;\n" : "=l"(p));
-  return p;
-}
-__device__ __forceinline__ uint64_t pol_evict_first() {
-  uint64_t p;
-  asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;\n" : "=l"(p));
-  return p;
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
@@ -590,409 +580,6 @@ __global__ void __launch_bounds__(512, 1) ccd_line_kernel(CcdArgs a) {
   cp_async_wait<0>();
 }
 
-// ---- warp-per-line fast path ------------------------------------------------------
-//
-// One warp solves one line: lane q owns rows [qR, qR+R) in registers.  The
-// chunk carries of the two block-Thomas sweeps are affine maps (M, v) that
-// compose as (M2, v2) o (M1, v1) = (M2 M1, v2 + M2 v1); a Kogge-Stone scan of
-// them over the 32 lanes (shuffles, no block barrier) gives every lane its
-// exact carry.  The tile of W lines is staged in shared memory by cp.async
-// (double-buffered) with one padding element per R rows, so lanes reading
-// rows R apart hit distinct banks; results are staged back for coalesced stores.
-
-template <typename T>
-struct Aff { T m0, m1, m2, m3, v0, v1; };
-
-template <typename T>
-__device__ __forceinline__ Aff<T> aff_compose(const Aff<T>& hi, const Aff<T>& lo) {
-  Aff<T> r;
-  r.m0 = hi.m0 * lo.m0 + hi.m1 * lo.m2;
-  r.m1 = hi.m0 * lo.m1 + hi.m1 * lo.m3;
-  r.m2 = hi.m2 * lo.m0 + hi.m3 * lo.m2;
-  r.m3 = hi.m2 * lo.m1 + hi.m3 * lo.m3;
-  r.v0 = hi.v0 + hi.m0 * lo.v0 + hi.m1 * lo.v1;
-  r.v1 = hi.v1 + hi.m2 * lo.v0 + hi.m3 * lo.v1;
-  return r;
-}
-
-template <typename T>
-__device__ __forceinline__ Aff<T> aff_shfl_up(const Aff<T>& a, int d) {
-  Aff<T> r;
-  r.m0 = __shfl_up_sync(0xffffffffu, a.m0, d); r.m1 = __shfl_up_sync(0xffffffffu, a.m1, d);
-  r.m2 = __shfl_up_sync(0xffffffffu, a.m2, d); r.m3 = __shfl_up_sync(0xffffffffu, a.m3, d);
-  r.v0 = __shfl_up_sync(0xffffffffu, a.v0, d); r.v1 = __shfl_up_sync(0xffffffffu, a.v1, d);
-  return r;
-}
-
-template <typename T>
-__device__ __forceinline__ Aff<T> aff_shfl_down(const Aff<T>& a, int d) {
-  Aff<T> r;
-  r.m0 = __shfl_down_sync(0xffffffffu, a.m0, d); r.m1 = __shfl_down_sync(0xffffffffu, a.m1, d);
-  r.m2 = __shfl_down_sync(0xffffffffu, a.m2, d); r.m3 = __shfl_down_sync(0xffffffffu, a.m3, d);
-  r.v0 = __shfl_down_sync(0xffffffffu, a.v0, d); r.v1 = __shfl_down_sync(0xffffffffu, a.v1, d);
-  return r;
-}
-
-template <typename T>
-__device__ __forceinline__ Aff<T> aff_identity() { return {T(1), T(0), T(0), T(1), T(0), T(0)}; }
-
-// copy tile t (TL lines) into fb[l*FSP + k + k/R]
-template <typename T, bool CONTIG, int R>
-__device__ __forceinline__ void issue_tile_padded(const CcdArgs& a, const T* __restrict__ f, T* fb, long long* lb,
-                                                  int t) {
-  const int TL = a.TL, n = a.n, FSP = a.FS;
-  const int64_t line0 = (int64_t)t * TL;
-  if (threadIdx.x < TL) {
-    const int64_t line = line0 + threadIdx.x;
-    long long b = -1;
-    if (line < a.n_lines) {
-      if (CONTIG) b = line * n;
-      else {
-        const int64_t o = line / a.inner, i = line - o * a.inner;
-        b = o * (int64_t)n * a.inner + i;
-      }
-    }
-    lb[threadIdx.x] = b;
-  }
-  __syncthreads();
-  const int total = TL * n;
-  if (CONTIG) {
-    // consecutive threads -> consecutive k of one line (coalesced)
-    int l = threadIdx.x / n, k = threadIdx.x - (threadIdx.x / n) * n;
-    const int step_l = blockDim.x / n, step_k = blockDim.x - step_l * n;
-    for (int e = threadIdx.x; e < total; e += blockDim.x) {
-      const long long b = lb[l];
-      cp_async<sizeof(T)>(fb + l * FSP + k + k / R, b >= 0 ? f + b + k : f, b >= 0);
-      l += step_l;
-      k += step_k;
-      if (k >= n) { k -= n; ++l; }
-    }
-  } else {
-    // consecutive threads -> consecutive lines at one k (coalesced)
-    for (int e = threadIdx.x; e < total; e += blockDim.x) {
-      const int k = e >> a.tl_shift, l = e & (TL - 1);
-      const long long b = lb[l];
-      cp_async<sizeof(T)>(fb + l * FSP + k + k / R, b >= 0 ? f + b + (int64_t)k * a.inner : f, b >= 0);
-    }
-  }
-  cp_async_commit();
-}
-
-// W warps per line: the line's rows are cut into 32 W chunks of R rows (lane
-// l of warp w of the line owns chunk 32 w + l); the carry scans run within
-// each warp by shuffles, then across the line's warps through shared memory.
-template <typename T, bool PERIODIC, bool CONTIG, int R, int W>
-__global__ void __launch_bounds__(256) ccd_warp_kernel(CcdArgs a) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int TL = a.TL, n = a.n, n_rows = a.n_rows, H0 = a.H0, FSP = a.FS;
-  const TabLayout lay{R, H0};
-  const int fsz = TL * FSP;
-  // shared: lbase(2 x TL) | tab | fbuf[nbuf] | sbuf
-  long long* lbase = reinterpret_cast<long long*>(smem_raw);
-  T* tab = reinterpret_cast<T*>(lbase + 2 * TL);
-  T* fbuf = tab + ((a.tab_total + 1) & ~1);
-  T* sbuf = fbuf + (size_t)a.nbuf * fsz;
-
-  const T* __restrict__ f = static_cast<const T*>(a.f);
-  const T* tabT = static_cast<const T*>(a.tabT);
-  stage_table<T>(tab, tabT, a.tab_total);
-
-  const int lane = threadIdx.x & 31;
-  const int wl = (threadIdx.x >> 5) / W;        // line of the tile owned by this warp
-  const int wq = (threadIdx.x >> 5) - wl * W;   // this warp's segment of the line
-  const int q = wq * 32 + lane;                 // chunk of the line owned by this lane
-  const int j0 = q * R;
-  const int cnt = max(0, min(R, n_rows - j0));  // rows of this lane
-  __shared__ Aff<T> s_tot[8 * W];               // per line of the tile (TL <= 8): warp totals
-  const T c1 = tab[lay.bc() + 30], c2 = tab[lay.bc() + 31];
-  const T* Lfi = tab + lay.cst();
-  const T Lf0 = Lfi[0], Lf1 = Lfi[1], Lf2 = Lfi[2], Lf3 = Lfi[3];
-  const T P0 = Lfi[4], P1 = Lfi[5], P2 = Lfi[6], P3 = Lfi[7];
-  const T H0m = Lfi[8], H1m = Lfi[9], H2m = Lfi[10], H3m = Lfi[11];
-  const T* Plast = Lfi + 12;
-  const T* Phi = tab + lay.phi();
-  const T* Psi = tab + lay.psi();
-  const T* head = tab + lay.head();
-  const double* tb = a.tab + lay.bc();
-  const double* J = a.J;
-  const bool in_head = !PERIODIC && j0 < H0;
-
-  int t = blockIdx.x;
-  int buf = 0;
-  if (t < a.n_tiles) issue_tile_padded<T, CONTIG, R>(a, f, fbuf, lbase, t);
-  for (; t < a.n_tiles; t += gridDim.x) {
-    const int tn = t + gridDim.x;
-    if (a.nbuf == 2 && tn < a.n_tiles) {
-      issue_tile_padded<T, CONTIG, R>(a, f, fbuf + (size_t)(buf ^ 1) * fsz, lbase + (buf ^ 1) * TL, tn);
-      cp_async_wait<1>();
-    } else {
-      if (a.nbuf == 1 && t != (int)blockIdx.x) issue_tile_padded<T, CONTIG, R>(a, f, fbuf, lbase, t);
-      cp_async_wait<0>();
-    }
-    __syncthreads();
-    T* fl = fbuf + (size_t)buf * fsz + wl * FSP;   // this warp's line (padded)
-    T* sl = sbuf + wl * FSP;
-    const long long* lb = lbase + buf * TL;
-    const bool valid = wl < TL && lb[wl] >= 0;
-    auto F = [&](int k) -> T { return fl[k + k / R]; };
-
-    if (wl < TL) {
-      // ---- closures (FP64, lanes 0 and last) --------------------------------
-      const int last = (n_rows - 1) / R;   // chunk holding the last row
-      double bl0 = 0.0, bl1 = 0.0, br0 = 0.0, br1 = 0.0;
-      if (!PERIODIC) {
-        if (q == 0) {
-          if (a.ovl) { bl0 = a.bcl0; bl1 = a.bcl1; }
-          else {
-            double fv[6];
-#pragma unroll
-            for (int k = 0; k < 6; ++k) fv[k] = (double)F(k);
-            bl0 = tb[16] * fv[0] + tb[17] * fv[1] + tb[18] * fv[2] + tb[19] * fv[3];
-            bl1 = tb[24] * fv[0] + tb[25] * fv[1] + tb[26] * fv[2] + tb[27] * fv[3] + tb[28] * fv[4] + tb[29] * fv[5];
-          }
-        }
-        if (q == last) {
-          if (a.ovr) { br0 = a.bcr0; br1 = a.bcr1; }
-          else {
-            double fv[6];
-#pragma unroll
-            for (int k = 0; k < 6; ++k) fv[k] = (double)F(n - 1 - k);
-            br0 = tb[20] * fv[0] + tb[21] * fv[1] + tb[22] * fv[2] + tb[23] * fv[3];
-            br1 = tb[24] * fv[0] + tb[25] * fv[1] + tb[26] * fv[2] + tb[27] * fv[3] + tb[28] * fv[4] + tb[29] * fv[5];
-          }
-        }
-      }
-      // ---- forward local sweep ------------------------------------------------
-      V2<T> y[R];
-      const int Nn = n - 1;
-      const int off = PERIODIC ? 0 : 1;
-      auto node = [&](int k) -> int {
-        if (PERIODIC) { if (k < 0) return k + Nn; if (k >= Nn) return k - Nn; }
-        return k;
-      };
-      V2<T> prev{T(0), T(0)};
-      if (cnt > 0) {
-        T fm = F(node(j0 + off - 1));
-        T f0 = F(node(j0 + off));
-#pragma unroll R
-        for (int r = 0; r < R; ++r) {
-          const int j = j0 + r;
-          if (r < cnt) {
-            const T fp = F(node(j + off + 1));
-            V2<T> b{c1 * (fp - fm), c2 * ((fm - T(2) * f0) + fp)};
-            if (!PERIODIC) {
-              if (j == 0) {
-                b.a = (T)((double)b.a - (tb[0] * bl0 + tb[1] * bl1));
-                b.b = (T)((double)b.b - (tb[2] * bl0 + tb[3] * bl1));
-              }
-              if (j == n_rows - 1) {
-                b.a = (T)((double)b.a - (tb[4] * br0 + tb[5] * br1));
-                b.b = (T)((double)b.b - (tb[6] * br0 + tb[7] * br1));
-              }
-            }
-            if (r == 0) {
-              prev = b;
-            } else if (in_head && j < H0) {
-              const V2<T> q = mv(head + 20 * j, prev);
-              prev = {b.a - q.a, b.b - q.b};
-            } else {
-              prev = {b.a - (Lf0 * prev.a + Lf1 * prev.b), b.b - (Lf2 * prev.a + Lf3 * prev.b)};
-            }
-            y[r] = prev;
-            fm = f0;
-            f0 = fp;
-          }
-        }
-      }
-      // ---- forward carry scan over lanes ---------------------------------------
-      {
-        Aff<T> m = aff_identity<T>();
-        if (cnt > 0) {
-          const int e = j0 + cnt;
-          const T* Tm = (in_head && e - 1 < H0) ? head + 20 * (e - 1) + 12 : Phi + 4 * (cnt - 1);
-          m = {Tm[0], Tm[1], Tm[2], Tm[3], prev.a, prev.b};
-        }
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-          const Aff<T> o = aff_shfl_up(m, d);
-          if (lane >= d) m = aff_compose(m, o);
-        }
-        Aff<T> ex = aff_shfl_up(m, 1);
-        if (lane == 0) ex = aff_identity<T>();
-        T l0 = __shfl_sync(0xffffffffu, m.v0, 31), l1 = __shfl_sync(0xffffffffu, m.v1, 31);
-        if (W > 1) {
-          // the warps before this one: P = total_{wq-1} o ... o total_0
-          if (lane == 31) s_tot[wl * W + wq] = m;
-          __syncthreads();
-          Aff<T> P = aff_identity<T>();
-          for (int v = 0; v < wq; ++v) P = aff_compose(s_tot[wl * W + v], P);
-          ex = aff_compose(ex, P);
-          Aff<T> all = P;
-          for (int v = wq; v < W; ++v) all = aff_compose(s_tot[wl * W + v], all);
-          l0 = all.v0;
-          l1 = all.v1;
-          __syncthreads();   // s_tot is reused by the backward scan
-        }
-        V2<T> Yin{ex.v0, ex.v1};
-        if (PERIODIC) {
-          // ring closure: Y_{-1} = Gf * (scan result of the last chunk)
-          const V2<T> ring = mv(Lfi + 16, V2<T>{l0, l1});
-          Yin = {ex.v0 + ex.m0 * ring.a + ex.m1 * ring.b, ex.v1 + ex.m2 * ring.a + ex.m3 * ring.b};
-        }
-        if ((PERIODIC || q > 0) && cnt > 0) {
-#pragma unroll R
-          for (int r = 0; r < R; ++r) {
-            const int j = j0 + r;
-            if (r < cnt) {
-              const T* mm = (in_head && j < H0) ? head + 20 * j + 12 : Phi + 4 * r;
-              y[r].a += mm[0] * Yin.a + mm[1] * Yin.b;
-              y[r].b += mm[2] * Yin.a + mm[3] * Yin.b;
-            }
-          }
-        }
-      }
-      // ---- backward local sweep -----------------------------------------------
-      V2<T> xn{T(0), T(0)};
-#pragma unroll R
-      for (int r = R - 1; r >= 0; --r) {
-        const int j = j0 + r;
-        if (r < cnt) {
-          V2<T> x;
-          if (in_head && j < H0) {
-            const V2<T> pp = mv(head + 20 * j + 4, y[r]);
-            const V2<T> qq = mv(head + 20 * j + 8, xn);
-            x = {pp.a - qq.a, pp.b - qq.b};
-          } else if (!PERIODIC && j == n_rows - 1) {
-            x = mv(Plast, y[r]);
-          } else {
-            x = {(P0 * y[r].a + P1 * y[r].b) - (H0m * xn.a + H1m * xn.b),
-                 (P2 * y[r].a + P3 * y[r].b) - (H2m * xn.a + H3m * xn.b)};
-          }
-          y[r] = x;
-          xn = x;
-        }
-      }
-      // ---- backward carry scan over lanes (suffix) -----------------------------------
-      {
-        Aff<T> m = aff_identity<T>();
-        if (cnt > 0) {
-          const T* Rm = (in_head && j0 < H0) ? head + 20 * j0 + 16 : Psi + 4 * cnt;
-          m = {Rm[0], Rm[1], Rm[2], Rm[3], xn.a, xn.b};
-        }
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-          const Aff<T> o = aff_shfl_down(m, d);
-          if (lane + d < 32) m = aff_compose(m, o);
-        }
-        Aff<T> ex = aff_shfl_down(m, 1);
-        if (lane == 31) ex = aff_identity<T>();
-        T l0 = __shfl_sync(0xffffffffu, m.v0, 0), l1 = __shfl_sync(0xffffffffu, m.v1, 0);
-        if (W > 1) {
-          // the warps after this one: Q = total_{wq+1} o ... o total_{W-1}
-          if (lane == 0) s_tot[wl * W + wq] = m;
-          __syncthreads();
-          Aff<T> Q = aff_identity<T>();
-          for (int v = W - 1; v > wq; --v) Q = aff_compose(s_tot[wl * W + v], Q);
-          ex = aff_compose(ex, Q);
-          Aff<T> all = Q;
-          for (int v = wq; v >= 0; --v) all = aff_compose(s_tot[wl * W + v], all);
-          l0 = all.v0;
-          l1 = all.v1;
-        }
-        V2<T> Xin{ex.v0, ex.v1};
-        if (PERIODIC) {
-          const V2<T> ring = mv(Lfi + 20, V2<T>{l0, l1});
-          Xin = {ex.v0 + ex.m0 * ring.a + ex.m1 * ring.b, ex.v1 + ex.m2 * ring.a + ex.m3 * ring.b};
-        }
-        if ((PERIODIC || q < last) && cnt > 0) {
-#pragma unroll R
-          for (int r = 0; r < R; ++r) {
-            const int j = j0 + r;
-            if (r < cnt) {
-              const T* mm = (in_head && j < H0) ? head + 20 * j + 16 : Psi + 4 * (cnt - r);
-              y[r].a += mm[0] * Xin.a + mm[1] * Xin.b;
-              y[r].b += mm[2] * Xin.a + mm[3] * Xin.b;
-            }
-          }
-        }
-      }
-      // ---- stage (d1, d2) in (own f line, sbuf line) --------------------------------------
-      __syncwarp();
-#pragma unroll R
-      for (int r = 0; r < R; ++r) {
-        if (r < cnt) {
-          const int k = PERIODIC ? j0 + r : j0 + r + 1;
-          fl[k + k / R] = y[r].a;
-          sl[k + k / R] = y[r].b;
-        }
-      }
-      if (!PERIODIC) {
-        if (q == 0 && cnt > 0) {
-          const double x0 = (double)y[0].a, x1 = (double)y[0].b;
-          fl[0] = (T)((tb[8] * x0 + tb[9] * x1) + bl0);
-          sl[0] = (T)((tb[10] * x0 + tb[11] * x1) + bl1);
-        }
-        if (q == last) {
-#pragma unroll R
-          for (int r = 0; r < R; ++r)
-            if (r == cnt - 1) {
-              const double x0 = (double)y[r].a, x1 = (double)y[r].b;
-              const int k = n - 1;
-              fl[k + k / R] = (T)((tb[12] * x0 + tb[13] * x1) + br0);
-              sl[k + k / R] = (T)((tb[14] * x0 + tb[15] * x1) + br1);
-            }
-        }
-      } else if (q == 0) {
-        const int k = n - 1;
-        fl[k + k / R] = y[0].a;
-        sl[k + k / R] = y[0].b;
-      }
-      (void)valid;
-    }
-    __syncthreads();
-    // ---- coalesced stores of the tile ---------------------------------------------------
-    {
-      const T* f1 = fbuf + (size_t)buf * fsz;
-      auto metric = [&](int k, double& o1, double& o2) {
-        if (J) {
-          const double Jk = J[k], dJk = J[n + k];
-          o2 = Jk * Jk * o2 + Jk * dJk * o1;
-          o1 = Jk * o1;
-        }
-      };
-      const int total = TL * n;
-      if (CONTIG) {
-        int l = threadIdx.x / n, k = threadIdx.x - (threadIdx.x / n) * n;
-        const int step_l = blockDim.x / n, step_k = blockDim.x - step_l * n;
-        for (int e = threadIdx.x; e < total; e += blockDim.x) {
-          const long long b = lb[l];
-          if (b >= 0) {
-            double o1 = (double)f1[l * FSP + k + k / R], o2 = (double)sbuf[l * FSP + k + k / R];
-            metric(k, o1, o2);
-            store_out<T>(a, b + k, o1, o2, k);
-          }
-          l += step_l;
-          k += step_k;
-          if (k >= n) { k -= n; ++l; }
-        }
-      } else {
-        for (int e = threadIdx.x; e < total; e += blockDim.x) {
-          const int k = e >> a.tl_shift, l = e & (TL - 1);
-          const long long b = lb[l];
-          if (b >= 0) {
-            double o1 = (double)f1[l * FSP + k + k / R], o2 = (double)sbuf[l * FSP + k + k / R];
-            metric(k, o1, o2);
-            store_out<T>(a, b + (int64_t)k * a.inner, o1, o2, k);
-          }
-        }
-      }
-    }
-    __syncthreads();
-    buf ^= (a.nbuf == 2) ? 1 : 0;
-  }
-  cp_async_wait<0>();
-}
-
 template <typename T>
 __global__ void wall_zero_kernel(T* g, int64_t outer, int64_t n, int64_t inner) {
   int64_t tot = outer * inner * 2;
@@ -1005,556 +592,98 @@ __global__ void wall_zero_kernel(T* g, int64_t outer, int64_t n, int64_t inner) 
   }
 }
 
+}  // namespace
+
+#include "ccd_chunk.cuh"
+
+namespace {
+
 // ---- host: factor tables ---------------------------------------------------
 
-// ---- lane-per-line kernel ---------------------------------------------------------
-//
-// For many lines (3-D grids): lane l of a warp owns line 32g + l and runs the
-// block-Thomas recurrences serially along it, so no scan, shuffle or carry
-// fix-up is needed.  A line is cut into chunks of kLaneCR rows and visited
-// twice:
-//   pass 1: forward sweep y_r = b_r - Lf_r y_{r-1}; the carry at the end of
-//           every chunk is kept in shared memory;
-//   pass 2: chunks in reverse order: the forward sweep of the chunk is redone
-//           from the stored carry (y in registers), then back substitution
-//           x_r = P_r y_r - H_r x_{r+1} from the carry of the chunk after it.
-// Each chunk's nodes (plus one halo node either side) are staged through a
-// [rows][lanes] shared tile so global loads and stores are coalesced for the
-// strided axes (lanes = adjacent lines) and the contiguous axis (lanes = nodes
-// of one line).  Periodic axes close the forward recurrence exactly on the
-// ring (Gf = (I - (-Lf)^N)^-1) and the backward one with the carry
-// X = Gb x_0, where x_0 of the zero-carry sweep is the sum over the first
-// kLaneK rows of (-H)^k P y_k (the neglected tail is below 0.46^64 of x_0).
-constexpr int kLaneCR = 16;
-constexpr int kLaneK = 64;
-
-struct LaneTab {
-  static constexpr int Lf = 0, P = 4, H = 8, Plast = 12, Gf = 16, Gb = 20, PhiC = 24, Q = 28, M = 32;
-  static constexpr int head = M + 4 * kLaneK;   // per head row: Lf, P, H (12)
-};
-
-template <typename T>
-__device__ __forceinline__ V2<T> mvs(const T* m, T a0, T a1) {
-  return {m[0] * a0 + m[1] * a1, m[2] * a0 + m[3] * a1};
+template <typename T, int R>
+ChunkConst<T, R> cast_chunk(const ChunkConst<double, R>& d) {
+  ChunkConst<T, R> o;
+  auto cp = [](const double* a, T* b, int n) { for (int k = 0; k < n; ++k) b[k] = (T)a[k]; };
+  cp(d.A, o.A, 4); cp(d.AR, o.AR, 4); cp(d.B, o.B, 4); cp(d.BR, o.BR, 4);
+  cp(d.P, o.P, 4); cp(d.Z, o.Z, 4); cp(d.Gf, o.Gf, 4); cp(d.Gb, o.Gb, 4); cp(d.AL, o.AL, 4); cp(d.BL, o.BL, 4);
+  cp(d.cl, o.cl, 4); cp(d.cr, o.cr, 4);
+  std::copy(d.Ml, d.Ml + 4, o.Ml); std::copy(d.Mr, d.Mr + 4, o.Mr);
+  std::copy(d.cIl, d.cIl + 4, o.cIl); std::copy(d.cIr, d.cIr + 4, o.cIr); std::copy(d.cII, d.cII + 6, o.cII);
+  return o;
 }
 
-// The lane table holds the factors in a scaled form: with D = diag(a1/h, a2/h^2)
-// the forward recurrence runs on y~ = D^-1 y, whose right-hand side is the
-// plain differences (f+ - f-, f- - 2 f0 + f+); every factor that touches y is
-// rescaled on the host (Lf~ = D^-1 Lf D, P~ = P D, ...), so no row pays for
-// the RHS constants.
-template <int N>
-__device__ __forceinline__ void cp_async_wait_dyn(int pending) {
-  // cp.async.wait_group takes an immediate: dispatch on the (small) count
-  if (pending <= 0) cp_async_wait<0>();
-  else if (pending == 1 || N <= 2) cp_async_wait<1>();
-  else cp_async_wait<2>();
-}
-
-template <typename T, bool PERIODIC, bool PLAIN, int NBUF, bool CONTIG>
-__global__ void __launch_bounds__(128) ccd_lane_kernel(CcdArgs a, const T* __restrict__ ltab_g, int ltab_total) {
-  constexpr int CR = kLaneCR, TR = CR + 2;
-  constexpr int TS = CONTIG ? 33 : 32;   // tile row stride (padded for the transposing copies)
-  constexpr int NT = NBUF + (CONTIG ? 1 : 0);   // + the d2 output tile
-  static_assert(NBUF == 2 || NBUF == 3, "f tile ring of 2 or 3 buffers");
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* lt = reinterpret_cast<T*>(smem_raw);
-  const int lt_pad = (ltab_total + 1) & ~1;
-  const int n = a.n, n_rows = a.n_rows, H0 = PERIODIC ? 0 : a.H0;
-  const int P = (n_rows + CR - 1) / CR;
-  const int warps = blockDim.x >> 5, wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  T* fb0 = lt + lt_pad + (size_t)wid * (NT * TR * TS + 64 * P);   // ring of f tiles [TR][TS]
-  T* dt = fb0 + NBUF * TR * TS;                                       // contiguous axis: d2 tile
-  T* cy = fb0 + NT * TR * TS;                                         // chunk-end carries [P][2][32]
-  stage_table<T>(lt, ltab_g, ltab_total);
-
-  const T* __restrict__ f = static_cast<const T*>(a.f);
-  const TabLayout lay{a.C, a.H0};
-  const double* tb = a.tab + lay.bc();
-  const double c1d = tb[30], c2d = tb[31];
-  const T lf0 = lt[LaneTab::Lf], lf1 = lt[LaneTab::Lf + 1], lf2 = lt[LaneTab::Lf + 2], lf3 = lt[LaneTab::Lf + 3];
-  const T p0 = lt[LaneTab::P], p1 = lt[LaneTab::P + 1], p2 = lt[LaneTab::P + 2], p3 = lt[LaneTab::P + 3];
-  const T h0 = lt[LaneTab::H], h1 = lt[LaneTab::H + 1], h2 = lt[LaneTab::H + 2], h3 = lt[LaneTab::H + 3];
-  const int Nn = n - 1;   // periodic: unique nodes
-  const int64_t inner = a.inner;
-  const int64_t n_groups = (a.n_lines + 31) / 32;
-  const double* J = a.J;
-
-  for (int64_t g = blockIdx.x * (int64_t)warps + wid; g < n_groups; g += (int64_t)gridDim.x * warps) {
-    const int64_t L = g * 32 + lane;
-    const bool act = L < a.n_lines;
-    int64_t base = 0;
-    if (act) {
-      const int64_t o = L / inner, i = L - o * inner;
-      base = o * (int64_t)n * inner + i;
-    }
-    const T* __restrict__ fl = f + base;
-    // asynchronous copy of nodes k0 + t, t in [0, KN), into tile[t][lane]
-    // FP64 strided axes: pass-1 chunks are staged with L2 evict_last (pass 2
-    // re-reads them), pass-2 chunks and the reused last chunk with
-    // evict_first (measured 2-3.5 % faster at 257^3; FP32 unchanged, so plain)
-    const uint64_t pol_keep = pol_evict_last(), pol_last = pol_evict_first();
-    auto stage = [&](T* tile, int k0, int KN, bool keep) {
-      if (CONTIG) {
-        // element e = (line ll, node t) of the chunk, e = lane + 32 i: runs of KN
-        // contiguous nodes per line, so each warp copy reads ~2 contiguous runs
-        int ll = lane / KN, t = lane - (lane / KN) * KN;
-        const int dl = 32 / KN, dt_ = 32 - dl * KN;
-        const T* fg = f + g * 32 * (int64_t)n;   // first line of the group
-        const int nl = (a.n_lines - g * 32 < 32) ? (int)(a.n_lines - g * 32) : 32;
-        const bool wrap = PERIODIC && (k0 < 0 || k0 + KN > Nn);
-        for (int i = 0; i < KN; ++i) {
-          if (ll < nl) {
-            int kk = k0 + t;
-            if (wrap) kk = (kk < 0) ? kk + Nn : (kk >= Nn ? kk - Nn : kk);
-            cp_async<sizeof(T)>(tile + t * TS + ll, fg + (ll * n + kk), true);
-          }
-          ll += dl;
-          t += dt_;
-          if (t >= KN) { t -= KN; ++ll; }
-        }
-        cp_async_commit();
-        return;
-      }
-      if (act) {
-        if (PERIODIC && (k0 < 0 || k0 + KN > Nn)) {
-          for (int t = 0; t < KN; ++t) {
-            int k = k0 + t;
-            k = (k < 0) ? k + Nn : (k >= Nn ? k - Nn : k);
-            cp_async<sizeof(T)>(tile + t * TS + lane, fl + (int64_t)k * inner, true);
-          }
-        } else {
-          const T* src = fl + (int64_t)k0 * inner;
-          if (sizeof(T) == 8) {
-            const uint64_t pol = keep ? pol_keep : pol_last;
-            for (int t = 0; t < KN; ++t) {
-              cp_async_pol<sizeof(T)>(tile + t * TS + lane, src, pol);
-              src += inner;
-            }
-          } else {
-            for (int t = 0; t < KN; ++t) {
-              cp_async<sizeof(T)>(tile + t * TS + lane, src, true);
-              src += inner;
-            }
-          }
-        }
-      }
-      cp_async_commit();
-    };
-    auto put = [&](int k, double o1, double o2) {
-      if (!act) return;
-      if (J) {
-        const double Jk = J[k], dJk = J[n + k];
-        o2 = Jk * Jk * o2 + Jk * dJk * o1;
-        o1 = Jk * o1;
-      }
-      store_out<T>(a, base + (int64_t)k * inner, o1, o2, k);
-    };
-    auto k0_of = [&](int c) { return PERIODIC ? c * CR - 1 : c * CR; };
-    auto cnt_of = [&](int c) { return min(CR, n_rows - c * CR); };
-
-    // chunk loads in visiting order: 0 .. P-1 (pass 1), then P-2 .. 0 (pass 2;
-    // chunk P-1 is reused from pass 1); load l lives in ring buffer l % NBUF
-    const int n_loads = 2 * P - 1;
-    auto chunk_of_load = [&](int l) { return l < P ? l : 2 * P - 2 - l; };
-    int issued = 0;
-    // make load `need` resident, keeping up to NBUF - 1 loads ahead in flight
-    auto acquire = [&](int need) -> const T* {
-      const int want = min(n_loads, need + NBUF);
-      while (issued < want) {
-        const int c = chunk_of_load(issued);
-        stage(fb0 + (issued % NBUF) * TR * TS, k0_of(c), cnt_of(c) + 2, issued < P - 1);
-        ++issued;
-      }
-      cp_async_wait_dyn<NBUF>(issued - need - 1);
-      __syncwarp();
-      return fb0 + (need % NBUF) * TR * TS;
-    };
-
-    // wall closures (FP64): boundary pieces bl, br and their (scaled) RHS corrections
-    double bl0 = 0.0, bl1 = 0.0, br0 = 0.0, br1 = 0.0;
-    T cl0 = T(0), cl1 = T(0), cr0 = T(0), cr1 = T(0);
-    if (!PERIODIC && act) {
-      if (a.ovl) { bl0 = a.bcl0; bl1 = a.bcl1; }
-      else {
-        double fv[6];
-#pragma unroll
-        for (int k = 0; k < 6; ++k) fv[k] = (double)fl[(int64_t)k * inner];
-        bl0 = tb[16] * fv[0] + tb[17] * fv[1] + tb[18] * fv[2] + tb[19] * fv[3];
-        bl1 = tb[24] * fv[0] + tb[25] * fv[1] + tb[26] * fv[2] + tb[27] * fv[3] + tb[28] * fv[4] + tb[29] * fv[5];
-      }
-      if (a.ovr) { br0 = a.bcr0; br1 = a.bcr1; }
-      else {
-        double fv[6];
-#pragma unroll
-        for (int k = 0; k < 6; ++k) fv[k] = (double)fl[(int64_t)(n - 1 - k) * inner];
-        br0 = tb[20] * fv[0] + tb[21] * fv[1] + tb[22] * fv[2] + tb[23] * fv[3];
-        br1 = tb[24] * fv[0] + tb[25] * fv[1] + tb[26] * fv[2] + tb[27] * fv[3] + tb[28] * fv[4] + tb[29] * fv[5];
-      }
-      cl0 = (T)((tb[0] * bl0 + tb[1] * bl1) / c1d);
-      cl1 = (T)((tb[2] * bl0 + tb[3] * bl1) / c2d);
-      cr0 = (T)((tb[4] * br0 + tb[5] * br1) / c1d);
-      cr1 = (T)((tb[6] * br0 + tb[7] * br1) / c2d);
-    }
-    // one forward row; SPECIAL rows carry closures / head factors / ring sums
-    auto row_fwd = [&](int r, T fm, T f0, T fp, V2<T> yp, bool special) -> V2<T> {
-      T ba = fp - fm, bb = (fm + fp) - T(2) * f0;
-      if (special) {
-        if (!PERIODIC) {
-          if (r == 0) { ba -= cl0; bb -= cl1; }
-          if (r == n_rows - 1) { ba -= cr0; bb -= cr1; }
-          if (r < H0) {
-            const T* m = lt + LaneTab::head + 12 * r;
-            return {ba - (m[0] * yp.a + m[1] * yp.b), bb - (m[2] * yp.a + m[3] * yp.b)};
-          }
-        }
-      }
-      return {ba - (lf0 * yp.a + lf1 * yp.b), bb - (lf2 * yp.a + lf3 * yp.b)};
-    };
-
-    // ---- pass 1: forward sweep, chunk-end carries -------------------------------------
-    V2<T> y{T(0), T(0)};
-    V2<T> acc{T(0), T(0)};   // periodic: sum_{k < K} (-H)^k P~ y~_k of the zero-carry sweep
-    for (int c = 0; c < P; ++c) {
-      const T* tile = acquire(c);
-      const int r0 = c * CR, cnt = cnt_of(c);
-      T fm = tile[lane], f0 = tile[TS + lane];
-      const bool special = cnt != CR || (PERIODIC ? (r0 < kLaneK) : (c == 0 || c == P - 1 || r0 < H0));
-      if (!special) {
-#pragma unroll
-        for (int q = 0; q < CR; ++q) {
-          const T fp = tile[(q + 2) * TS + lane];
-          y = row_fwd(r0 + q, fm, f0, fp, y, false);
-          fm = f0;
-          f0 = fp;
-        }
-      } else {
-        for (int q = 0; q < cnt; ++q) {
-          const int r = r0 + q;
-          const T fp = tile[(q + 2) * TS + lane];
-          y = row_fwd(r, fm, f0, fp, y, true);
-          if (PERIODIC && r < kLaneK) {
-            const V2<T> u = mvs(lt + LaneTab::M + 4 * r, y.a, y.b);
-            acc.a += u.a;
-            acc.b += u.b;
-          }
-          fm = f0;
-          f0 = fp;
-        }
-      }
-      cy[(c * 2) * 32 + lane] = y.a;
-      cy[(c * 2 + 1) * 32 + lane] = y.b;
-      __syncwarp();
-    }
-    // ---- ring closures -------------------------------------------------------------
-    V2<T> yin{T(0), T(0)}, xc{T(0), T(0)};
-    if (PERIODIC) {
-      yin = mvs(lt + LaneTab::Gf, y.a, y.b);
-      V2<T> corr = yin;
-      for (int c = 0; c + 1 < P; ++c) {
-        corr = mvs(lt + LaneTab::PhiC, corr.a, corr.b);
-        cy[(c * 2) * 32 + lane] += corr.a;
-        cy[(c * 2 + 1) * 32 + lane] += corr.b;
-      }
-      const V2<T> qy = mvs(lt + LaneTab::Q, yin.a, yin.b);
-      xc = mvs(lt + LaneTab::Gb, acc.a + qy.a, acc.b + qy.b);
-      __syncwarp();
-    }
-    // ---- pass 2: chunks in reverse order ------------------------------------------------
-    const int noff = PERIODIC ? 0 : 1;   // node of row r
-    for (int c = P - 1; c >= 0; --c) {
-      const T* tile = acquire(c == P - 1 ? P - 1 : 2 * P - 2 - c);
-      const int r0 = c * CR, cnt = cnt_of(c);
-      const bool special = !PERIODIC && (c == 0 || c == P - 1 || r0 < H0);
-      V2<T> yr[CR];
-      V2<T> xlast{T(0), T(0)};
-      V2<T> yp = (c == 0) ? yin : V2<T>{cy[((c - 1) * 2) * 32 + lane], cy[((c - 1) * 2 + 1) * 32 + lane]};
-      T fm = tile[lane], f0 = tile[TS + lane];
-      if (!special && cnt == CR) {
-#pragma unroll
-        for (int q = 0; q < CR; ++q) {
-          const T fp = tile[(q + 2) * TS + lane];
-          yp = row_fwd(r0 + q, fm, f0, fp, yp, false);
-          yr[q] = yp;
-          fm = f0;
-          f0 = fp;
-        }
-        __syncwarp();   // the tile is refilled by the prefetch after next
-#pragma unroll
-        for (int q = CR - 1; q >= 0; --q) {
-          const V2<T> x{(p0 * yr[q].a + p1 * yr[q].b) - (h0 * xc.a + h1 * xc.b),
-                        (p2 * yr[q].a + p3 * yr[q].b) - (h2 * xc.a + h3 * xc.b)};
-          xc = x;
-          yr[q] = x;
-        }
-      } else {
-#pragma unroll
-        for (int q = 0; q < CR; ++q) {
-          if (q < cnt) {
-            const T fp = tile[(q + 2) * TS + lane];
-            yp = row_fwd(r0 + q, fm, f0, fp, yp, true);
-            yr[q] = yp;
-            fm = f0;
-            f0 = fp;
-          }
-        }
-        __syncwarp();
-#pragma unroll
-        for (int q = CR - 1; q >= 0; --q) {
-          if (q < cnt) {
-            const int r = r0 + q;
-            V2<T> x;
-            if (!PERIODIC && r == n_rows - 1) {
-              x = mvs(lt + LaneTab::Plast, yr[q].a, yr[q].b);
-              xlast = x;
-            } else if (r < H0) {
-              const T* pm = lt + LaneTab::head + 12 * r + 4;
-              const T* hm = pm + 4;
-              x = {(pm[0] * yr[q].a + pm[1] * yr[q].b) - (hm[0] * xc.a + hm[1] * xc.b),
-                   (pm[2] * yr[q].a + pm[3] * yr[q].b) - (hm[2] * xc.a + hm[3] * xc.b)};
-            } else {
-              x = {(p0 * yr[q].a + p1 * yr[q].b) - (h0 * xc.a + h1 * xc.b),
-                   (p2 * yr[q].a + p3 * yr[q].b) - (h2 * xc.a + h3 * xc.b)};
-            }
-            xc = x;
-            yr[q] = x;
-          }
-        }
-      }
-      if (CONTIG) {
-        // results through the (consumed) f tile and the d2 tile, then runs of
-        // contiguous nodes per line
-        T* ot = const_cast<T*>(tile);
-#pragma unroll
-        for (int q = 0; q < CR; ++q) {
-          if (q < cnt) {
-            ot[(q + 1) * TS + lane] = yr[q].a;
-            dt[(q + 1) * TS + lane] = yr[q].b;
-          }
-        }
-        int t0 = 1, t1 = cnt + 1;
-        if (!PERIODIC && c == P - 1) {
-          const double x0 = (double)xlast.a, x1 = (double)xlast.b;
-          ot[(cnt + 1) * TS + lane] = (T)((tb[12] * x0 + tb[13] * x1) + br0);
-          dt[(cnt + 1) * TS + lane] = (T)((tb[14] * x0 + tb[15] * x1) + br1);
-          t1 = cnt + 2;
-        }
-        if (!PERIODIC && c == 0) {
-          const double x0 = (double)xc.a, x1 = (double)xc.b;
-          ot[lane] = (T)((tb[8] * x0 + tb[9] * x1) + bl0);
-          dt[lane] = (T)((tb[10] * x0 + tb[11] * x1) + bl1);
-          t0 = 0;
-        }
-        __syncwarp();
-        const int KN = t1 - t0;
-        const int k0 = k0_of(c) + t0;
-        int ll = lane / KN, t = lane - (lane / KN) * KN;
-        const int dl = 32 / KN, dt_ = 32 - dl * KN;
-        const int64_t g0 = g * 32 * (int64_t)n;
-        const int nl = (a.n_lines - g * 32 < 32) ? (int)(a.n_lines - g * 32) : 32;
-        const bool plain_c = a.d1 && a.d2 && !a.vd_out && !J;
-        T* o1p = static_cast<T*>(a.d1) + g0;
-        T* o2p = static_cast<T*>(a.d2) + g0;
-        if (a.cr_out) {
-          // corrector epilogue: all of this run's u* and rho first, then the
-          // stores (see the strided branch)
-          double pu[CR + 2], pr[CR + 2];
-          int l2 = ll, t2 = t;
-#pragma unroll
-          for (int i = 0; i < CR + 2; ++i) {
-            pu[i] = 0.0;
-            pr[i] = 1.0;
-            if (i < KN && l2 < nl) {
-              const int64_t gi = g0 + (int64_t)l2 * n + k0 + t2;
-              pu[i] = (double)static_cast<const T*>(a.cr_u)[gi];
-              pr[i] = (double)static_cast<const T*>(a.cr_rho)[gi];
-            }
-            l2 += dl;
-            t2 += dt_;
-            if (t2 >= KN) { t2 -= KN; ++l2; }
-          }
-#pragma unroll
-          for (int i = 0; i < CR + 2; ++i) {
-            if (i < KN && ll < nl) {
-              const int node = k0 + t;
-              double o1 = (double)ot[(t0 + t) * TS + ll];
-              if (J) o1 = J[node] * o1;
-              double v = pu[i];
-              if (!(a.cr_wall && (node == 0 || node == n - 1))) v = __dsub_rn(pu[i], __dmul_rn(a.cr_dt / pr[i], o1));
-              static_cast<T*>(a.cr_out)[g0 + (int64_t)ll * n + node] = (T)v;
-            }
-            ll += dl;
-            t += dt_;
-            if (t >= KN) { t -= KN; ++ll; }
-          }
-        } else if (a.vd_out) {
-          // variable-density epilogue: operands first, then the stores
-          double pr[CR + 2], pdr[CR + 2], po[CR + 2];
-          int l2 = ll, t2 = t;
-#pragma unroll
-          for (int i = 0; i < CR + 2; ++i) {
-            pr[i] = 1.0;
-            pdr[i] = 0.0;
-            po[i] = 0.0;
-            if (i < KN && l2 < nl) {
-              const int64_t gi = g0 + (int64_t)l2 * n + k0 + t2;
-              pr[i] = (double)static_cast<const T*>(a.vd_rho)[gi];
-              pdr[i] = (double)static_cast<const T*>(a.vd_drho)[gi];
-              if (a.vd_accumulate) po[i] = (double)static_cast<const T*>(a.vd_out)[gi];
-            }
-            l2 += dl;
-            t2 += dt_;
-            if (t2 >= KN) { t2 -= KN; ++l2; }
-          }
-#pragma unroll
-          for (int i = 0; i < CR + 2; ++i) {
-            if (i < KN && ll < nl) {
-              const int node = k0 + t;
-              double o1 = (double)ot[(t0 + t) * TS + ll], o2 = (double)dt[(t0 + t) * TS + ll];
-              if (J) {
-                const double Jk = J[node], dJk = J[n + node];
-                o2 = Jk * Jk * o2 + Jk * dJk * o1;
-                o1 = Jk * o1;
-              }
-              const double r = pr[i];
-              double tv = o2 / r - (pdr[i] / (r * r)) * o1;
-              if (a.vd_accumulate) tv = po[i] + tv;
-              static_cast<T*>(a.vd_out)[g0 + (int64_t)ll * n + node] = (T)tv;
-            }
-            ll += dl;
-            t += dt_;
-            if (t >= KN) { t -= KN; ++ll; }
-          }
-        } else
-        for (int i = 0; i < KN; ++i) {
-          if (ll < nl) {
-            const int node = k0 + t;
-            const T v1 = ot[(t0 + t) * TS + ll], v2 = dt[(t0 + t) * TS + ll];
-            if (plain_c) {
-              o1p[ll * n + node] = v1;
-              o2p[ll * n + node] = v2;
-            } else {
-              double o1 = (double)v1, o2 = (double)v2;
-              if (J) {
-                const double Jk = J[node], dJk = J[n + node];
-                o2 = Jk * Jk * o2 + Jk * dJk * o1;
-                o1 = Jk * o1;
-              }
-              store_out<T>(a, g0 + (int64_t)ll * n + node, o1, o2, node);
-            }
-          }
-          ll += dl;
-          t += dt_;
-          if (t >= KN) { t -= KN; ++ll; }
-        }
-        if (PERIODIC && c == 0) put(Nn, (double)xc.a, (double)xc.b);   // image node N = node 0 (own line)
-        __syncwarp();
-        continue;
-      }
-      // ascending burst of coalesced stores (lanes = adjacent lines)
-      if (PLAIN) {
-        if (act) {
-          T* o1 = static_cast<T*>(a.d1) + base + (int64_t)(r0 + noff) * inner;
-          T* o2 = static_cast<T*>(a.d2) + base + (int64_t)(r0 + noff) * inner;
-#pragma unroll
-          for (int q = 0; q < CR; ++q) {
-            if (q < cnt) {
-              __stcs(o1, yr[q].a);   // streaming: keep L2 for the lines pass 2 re-reads
-              __stcs(o2, yr[q].b);
-              o1 += inner;
-              o2 += inner;
-            }
-          }
-        }
-      } else if (a.cr_out) {
-        // corrector epilogue: the chunk's u* and rho are loaded before any
-        // store (the stores may alias u*, which would otherwise serialize each
-        // node's loads behind the previous node's store)
-        if (act) {
-          const int64_t o0 = base + (int64_t)(r0 + noff) * inner;
-          const T* cu = static_cast<const T*>(a.cr_u) + o0;
-          const T* crh = static_cast<const T*>(a.cr_rho) + o0;
-          T* co = static_cast<T*>(a.cr_out) + o0;
-          double pu[CR], pr[CR];
-#pragma unroll
-          for (int q = 0; q < CR; ++q) {
-            pu[q] = 0.0;
-            pr[q] = 1.0;
-            if (q < cnt) {
-              pu[q] = (double)cu[(int64_t)q * inner];
-              pr[q] = (double)crh[(int64_t)q * inner];
-            }
-          }
-#pragma unroll
-          for (int q = 0; q < CR; ++q) {
-            if (q < cnt) {
-              const int k = r0 + q + noff;
-              double o1 = (double)yr[q].a;
-              if (J) o1 = J[k] * o1;
-              double v = pu[q];
-              if (!(a.cr_wall && (k == 0 || k == n - 1))) v = __dsub_rn(pu[q], __dmul_rn(a.cr_dt / pr[q], o1));
-              co[(int64_t)q * inner] = (T)v;
-            }
-          }
-        }
-      } else if (a.vd_out) {
-        // variable-density epilogue: operands first, then the stores (as above)
-        if (act) {
-          const int64_t o0 = base + (int64_t)(r0 + noff) * inner;
-          const T* vr = static_cast<const T*>(a.vd_rho) + o0;
-          const T* vdr = static_cast<const T*>(a.vd_drho) + o0;
-          T* vo = static_cast<T*>(a.vd_out) + o0;
-          double pr[CR], pdr[CR], po[CR];
-#pragma unroll
-          for (int q = 0; q < CR; ++q) {
-            pr[q] = 1.0;
-            pdr[q] = 0.0;
-            po[q] = 0.0;
-            if (q < cnt) {
-              pr[q] = (double)vr[(int64_t)q * inner];
-              pdr[q] = (double)vdr[(int64_t)q * inner];
-              if (a.vd_accumulate) po[q] = (double)vo[(int64_t)q * inner];
-            }
-          }
-#pragma unroll
-          for (int q = 0; q < CR; ++q) {
-            if (q < cnt) {
-              const int k = r0 + q + noff;
-              double o1 = (double)yr[q].a, o2 = (double)yr[q].b;
-              if (J) {
-                const double Jk = J[k], dJk = J[n + k];
-                o2 = Jk * Jk * o2 + Jk * dJk * o1;
-                o1 = Jk * o1;
-              }
-              const double r = pr[q];
-              double tv = o2 / r - (pdr[q] / (r * r)) * o1;
-              if (a.vd_accumulate) tv = po[q] + tv;
-              vo[(int64_t)q * inner] = (T)tv;
-            }
-          }
-        }
-      } else {
-#pragma unroll
-        for (int q = 0; q < CR; ++q)
-          if (q < cnt) put(r0 + q + noff, (double)yr[q].a, (double)yr[q].b);
-      }
-      if (!PERIODIC && c == P - 1) {
-        const double x0 = (double)xlast.a, x1 = (double)xlast.b;
-        put(n - 1, (tb[12] * x0 + tb[13] * x1) + br0, (tb[14] * x0 + tb[15] * x1) + br1);
-      }
-      if (c == 0) {
-        if (!PERIODIC) {
-          const double x0 = (double)xc.a, x1 = (double)xc.b;
-          put(0, (tb[8] * x0 + tb[9] * x1) + bl0, (tb[10] * x0 + tb[11] * x1) + bl1);
-        } else {
-          put(Nn, (double)xc.a, (double)xc.b);   // image node N = node 0
-        }
-      }
-      __syncwarp();   // this tile may be refilled by the next acquire
-    }
-    cp_async_wait<0>();
-    __syncwarp();
+// constants of the chunk kernels (see ccd_chunk.cuh); G: the wall table, rows
+// beyond kChunkHead or beyond the line are 0
+template <int R>
+ChunkConst<double, R> chunk_tables(const tpf_ccd_plan* p, std::vector<double>& G) {
+  const double h = p->h;
+  const int n_rows = p->n_rows;
+  const M2 L = {kAlpha1, kB1 * h, kB2 / h, kBeta2};
+  const M2 U = {kAlpha1, -kB1 * h, -kB2 / h, kBeta2};
+  const M2 Ml = {-1.5, 1.5 * h, 0.0, 0.0};
+  const M2 Mr = {-1.5, -1.5 * h, 0.0, 0.0};
+  M2 S = eye();   // fixed point of S = I - L S^-1 U
+  for (int it = 0; it < 400; ++it) S = sub(eye(), mul(mul(L, inv(S)), U));
+  const M2 P = inv(S), A = neg(mul(L, P)), B = neg(mul(P, U));
+  const double d[2] = {kA1 / h, kA2 / (h * h)};
+  auto sim = [&](const M2& m) { return M2{m[0], m[1] * d[1] / d[0], m[2] * d[0] / d[1], m[3]}; };   // D^-1 m D
+  auto rmul = [&](const M2& m) { return M2{m[0] * d[0], m[1] * d[1], m[2] * d[0], m[3] * d[1]}; };  // m D
+  ChunkConst<double, R> K{};
+  G.assign(4 * (kChunkHead + R), 0.0);
+  auto set = [](double* o, const M2& m) { for (int k = 0; k < 4; ++k) o[k] = m[k]; };
+  M2 pa = eye(), pb = eye();
+  for (int r = 0; r < R; ++r) {
+    pa = mul(A, pa);
+    pb = mul(B, pb);
   }
+  set(K.A, sim(A));
+  set(K.AR, sim(pa));
+  set(K.B, B);
+  set(K.BR, pb);
+  set(K.P, rmul(P));
+  set(K.Ml, Ml);
+  set(K.Mr, Mr);
+  const double cIl[4] = {-23.0 / 6.0, 21.0 / 4.0, -1.5, 1.0 / 12.0};
+  const double cII[6] = {45.0, -154.0, 214.0, -156.0, 61.0, -10.0};
+  for (int q = 0; q < 4; ++q) {
+    K.cIl[q] = cIl[q] / h;
+    K.cIr[q] = -cIl[q] / h;
+  }
+  for (int q = 0; q < 6; ++q) K.cII[q] = cII[q] / (12.0 * h * h);
+  set(K.cl, {L[0] / d[0], L[1] / d[0], L[2] / d[1], L[3] / d[1]});
+  if (p->bc == TPF_BC_WALL) {
+    // the last pivot, and M^-1 e_0 by the two sweeps
+    const M2 Sl = add(sub(eye(), mul(neg(A), U)), mul(U, Mr)), Pl = inv(Sl);
+    set(K.Z, mul(Pl, S));
+    set(K.cr, mul(Pl, U));
+    std::vector<M2> V(n_rows);
+    M2 y = eye();
+    for (int j = 0; j < n_rows; ++j) {
+      V[j] = y;
+      y = mul(A, y);
+    }
+    V[n_rows - 1] = mul(Pl, V[n_rows - 1]);
+    for (int j = n_rows - 2; j >= 0; --j) V[j] = add(mul(P, V[j]), mul(B, V[j + 1]));
+    const M2 B0 = sub(add(eye(), mul(L, Ml)), S);
+    const M2 Kg = mul(B0, inv(add(eye(), mul(V[0], B0))));
+    for (int j = 0; j < std::min(n_rows, kChunkHead); ++j) set(G.data() + 4 * j, mul(V[j], Kg));
+  } else {
+    const int Q = (n_rows + R - 1) / R, len = n_rows - (Q - 1) * R;
+    M2 an = eye(), bn = eye(), al = eye(), bl = eye();
+    for (int k = 0; k < n_rows; ++k) {
+      an = mul(A, an);
+      bn = mul(B, bn);
+      if (k == len - 1) {
+        al = an;
+        bl = bn;
+      }
+    }
+    set(K.Gf, sim(inv(sub(eye(), an))));
+    set(K.Gb, inv(sub(eye(), bn)));
+    set(K.AL, sim(al));
+    set(K.BL, bl);
+  }
+  return K;
 }
 
 int build_tables(tpf_ccd_plan* p, std::vector<double>& tab) {
@@ -1689,63 +818,6 @@ int build_tables(tpf_ccd_plan* p, std::vector<double>& tab) {
   tab[b + 31] = kA2 / (h * h);
   p->P = P;
   p->H0 = H0;
-  // lane-per-line kernel table, scaled by D = diag(a1/h, a2/h^2) (see ccd_lane_kernel)
-  {
-    const double d[2] = {kA1 / h, kA2 / (h * h)};
-    auto sim = [&](const M2& m) {   // D^-1 m D
-      return M2{m[0], m[1] * d[1] / d[0], m[2] * d[0] / d[1], m[3]};
-    };
-    auto rmul = [&](const M2& m) {  // m D
-      return M2{m[0] * d[0], m[1] * d[1], m[2] * d[0], m[3] * d[1]};
-    };
-    const int tot = LaneTab::head + 12 * H0;
-    std::vector<double>& lt = p->ltab_host;
-    lt.assign(tot, 0.0);
-    const M2 Lfs = sim(Lfinf), Ps = rmul(Pinf);
-    for (int q = 0; q < 4; ++q) {
-      lt[LaneTab::Lf + q] = Lfs[q];
-      lt[LaneTab::P + q] = Ps[q];
-      lt[LaneTab::H + q] = Hinf[q];
-    }
-    if (p->bc == TPF_BC_WALL) {
-      const M2 Pl = rmul(Pm[n_rows - 1]);
-      for (int q = 0; q < 4; ++q) lt[LaneTab::Plast + q] = Pl[q];
-      for (int j = 0; j < H0; ++j) {
-        const M2 lj = sim(Lf[j]), pj = rmul(Pm[j]);
-        for (int q = 0; q < 4; ++q) {
-          lt[LaneTab::head + 12 * j + q] = lj[q];
-          lt[LaneTab::head + 12 * j + 4 + q] = pj[q];
-          lt[LaneTab::head + 12 * j + 8 + q] = Hm[j][q];
-        }
-      }
-    } else {
-      // ring: Tr = (-Lf)^N, Rr = (-H)^N; PhiC = (-Lf)^CR; M_k = (-H)^k P; Q = sum_k M_k (-Lf)^(k+1)
-      M2 Tr = eye(), Rr = eye(), PhiC = eye();
-      for (int k = 0; k < n_rows; ++k) {
-        Tr = mul(neg(Lfinf), Tr);
-        Rr = mul(neg(Hinf), Rr);
-      }
-      for (int k = 0; k < kLaneCR; ++k) PhiC = mul(neg(Lfinf), PhiC);
-      const M2 Gf = inv(sub(eye(), Tr)), Gb = inv(sub(eye(), Rr));
-      M2 Hk = eye(), Phk = eye(), Q = {0, 0, 0, 0};
-      const int K = std::min(kLaneK, n_rows);
-      for (int k = 0; k < K; ++k) {
-        const M2 Mk = mul(Hk, Pinf);
-        Phk = mul(neg(Lfinf), Phk);
-        Q = add(Q, mul(Mk, Phk));
-        const M2 Mks = rmul(Mk);
-        for (int q = 0; q < 4; ++q) lt[LaneTab::M + 4 * k + q] = Mks[q];
-        Hk = mul(neg(Hinf), Hk);
-      }
-      const M2 Gfs = sim(Gf), PhiCs = sim(PhiC), Qs = rmul(Q);
-      for (int q = 0; q < 4; ++q) {
-        lt[LaneTab::Gf + q] = Gfs[q];
-        lt[LaneTab::Gb + q] = Gb[q];
-        lt[LaneTab::PhiC + q] = PhiCs[q];
-        lt[LaneTab::Q + q] = Qs[q];
-      }
-    }
-  }
   return TPF_OK;
 }
 
@@ -1798,164 +870,107 @@ LaunchShape pick_shape(const tpf_ccd_plan* p, bool contig, int64_t n_lines) {
   return best;
 }
 
-template <typename T, int R>
-LaunchShape pick_warp_shape(const tpf_ccd_plan* p, int64_t n_lines, int W) {
-  const int n = (int)p->n_pts;
-  int FSP = n + (n - 1) / R + 1;
-  if (FSP % 2 == 0) ++FSP;
-  const int nsm = tpf::sm_count();
-  const int regs = R == 8 ? 128 : (R == 16 ? 168 : 255);
-  TabLayout lay{R, p->H0};
-  LaunchShape best{};
-  best.TL = 0;
-  double best_score = -1e30;
-  const int tl_opts[4] = {8, 4, 2, 1};
-  for (int t = 0; t < 4; ++t) {
-    const int TL = tl_opts[t];
-    const int threads = 32 * W * TL;
-    if (threads > 256) continue;
-    const int64_t tiles = (n_lines + TL - 1) / TL;
-    const size_t fsz = (size_t)TL * FSP;
-    for (int nbuf = 2; nbuf >= 1; --nbuf) {
-      const size_t sm = sizeof(long long) * 2 * TL + sizeof(T) * (((size_t)lay.total() + 1) & ~(size_t)1) +
-                        sizeof(T) * (nbuf + 1) * fsz + 64;
-      if (sm > 225 * 1024) continue;
-      const int by_smem = (int)((228 * 1024) / (sm + 1024));
-      const int by_regs = 65536 / (regs * threads);
-      const int per_sm = std::max(1, std::min(std::min(by_smem, by_regs), 16));
-      const int64_t grid = std::min<int64_t>(tiles, (int64_t)nsm * per_sm);
-      const double waves = (double)tiles / (double)grid;
-      double score = 400.0 * std::min(1.0, (double)grid / nsm) + 0.25 * std::min(per_sm * threads, 2048) +
-                     (nbuf == 2 && waves > 1.5 ? 150.0 : 0.0) - (nbuf == 2 && waves <= 1.0 ? 300.0 : 0.0);
-      if (score > best_score) {
-        best_score = score;
-        best = {TL, 0, FSP, nbuf, (int)grid, sm};
-      }
-    }
+// ---- chunk kernels: launch -------------------------------------------------------
+// How a call's lines are cut up: TL adjacent lines per block (0: a line is too
+// long for a block), `staged` for the strided axes, `pitch` of the contiguous
+// axis' lines in shared memory.  The results do not depend on any of them (each
+// line is solved by its own threads).
+struct ChunkShape {
+  int TL, threads, pitch;
+  bool staged;
+  size_t smem;
+  unsigned blocks;
+};
+
+// The rule (one B200, FP64 unless said; us per call):
+// * Strided axes: 16 lines, i.e. 128-byte rows; 32 where that keeps as many
+//   threads resident and the rows do not start on 32-byte sectors (257^3: 98.8
+//   against 108.9 on axis 0; 256^3 nodes, whose rows do: 89.0 against 81.7;
+//   129 x 97 x 162 axis 1, 480 resident threads against 384: 13.1 against 16.3).
+// * Contiguous axis: 8 or 16 lines, whichever keeps more threads resident (193
+//   nodes: 45.3 with 8, 54.5 with 16; 162 nodes: 18.6 and 15.3).
+// * Fewer lines per block while that leaves half of the SMs without one, down
+//   to 128 threads (401 x 301: 6.2 with 8 lines, 7.6 with 16).
+// * Staging (the next tile's f copied while this one is solved) in FP64 once
+//   every resident block has more than two tiles: 257^3 98.8 against 112.5,
+//   193^3 45.3 against 57.9; 129 x 97 x 162 the other way, 14.1 against 13.1;
+//   FP32 191 x 160 x 225 29.5 against 19.6.
+template <typename T>
+ChunkShape chunk_shape(const tpf_ccd_plan* p, bool contig, int64_t n_lines, int64_t inner) {
+  constexpr bool F64 = std::is_same<T, double>::value;
+  const int Q = (p->n_rows + kChunkR - 1) / kChunkR, n = (int)p->n_pts, nsm = tpf::sm_count();
+  ChunkShape s{};
+  // a pitch of n has bank conflicts of degree gcd(n, 16) (FP64; FP32 gcd(n, 32))
+  s.pitch = (n & 3) == 0 ? n + 1 : n;
+  const size_t fixed = 4 * (size_t)(kChunkHead + kChunkR);
+  auto threads = [&](int tl) { return (tl * Q + 31) / 32 * 32; };
+  auto smem = [&](int tl, bool staged) {
+    const size_t tiles = contig ? 2 * (((size_t)tl * s.pitch + 3) & ~(size_t)3) : staged ? (size_t)tl * n : 0;
+    return sizeof(T) * (fixed + 4 * (size_t)threads(tl) + tl + tiles);
+  };
+  const size_t limit = 200 * 1024;
+  auto fits = [&](int tl) { return tl * Q <= 512 && smem(tl, false) <= limit; };
+  auto per_sm = [&](int tl) { return std::max(1, 65536 / ((F64 ? 128 : 96) * threads(tl))); };
+  auto resident = [&](int tl) { return fits(tl) ? per_sm(tl) * tl * Q : 0; };
+  auto tiles = [&](int tl) { return (n_lines + tl - 1) / tl; };
+  int TL = 16;
+  if (contig) TL = resident(16) > resident(8) ? 16 : 8;
+  else if (resident(32) >= resident(16) && (inner * sizeof(T)) % 32 != 0 && tiles(32) >= nsm) TL = 32;
+  while (TL > 2 && !fits(TL)) TL >>= 1;
+  if (!fits(TL)) return s;
+  while (TL > 2 && 2 * tiles(TL) <= nsm && TL / 2 * Q >= 128) TL >>= 1;
+  s.TL = TL;
+  s.threads = threads(TL);
+  const int64_t slots = (int64_t)nsm * per_sm(TL);
+  s.staged = !contig && F64 && tiles(TL) > 2 * slots && smem(TL, true) <= limit;
+  s.smem = smem(TL, s.staged);
+  s.blocks = (unsigned)(s.staged ? slots : tiles(TL));
+  return s;
+}
+
+template <typename T>
+int launch_chunk(const tpf_ccd_plan* p, CcdArgs a, bool per, bool contig, const ChunkShape& sh, cudaStream_t s) {
+  const int Q = (p->n_rows + kChunkR - 1) / kChunkR;
+  a.TL = sh.TL;
+  a.tl_shift = 0;
+  while ((1 << a.tl_shift) < sh.TL) ++a.tl_shift;
+  a.n_tiles = (int)((a.n_lines + sh.TL - 1) / sh.TL);
+  const T* g;
+  const ChunkConst<T, kChunkR>* K;
+  if constexpr (std::is_same<T, double>::value) {
+    g = p->d_g64;
+    K = &p->c64;
+  } else {
+    g = p->d_g32;
+    K = &p->c32;
   }
-  return best;
-}
-
-// launch shape of the warp kernel for one (lines per block, tile buffers) choice
-template <typename T, int R>
-LaunchShape warp_shape(const tpf_ccd_plan* p, int64_t n_lines, int W, int TL, int nbuf) {
-  const int n = (int)p->n_pts;
-  int FSP = n + (n - 1) / R + 1;
-  if (FSP % 2 == 0) ++FSP;
-  const int nsm = tpf::sm_count();
-  const int regs = R == 8 ? 128 : (R == 16 ? 168 : 255);
-  TabLayout lay{R, p->H0};
-  LaunchShape out{};
-  out.TL = 0;
-  const int threads = 32 * W * TL;
-  if (threads > 256) return out;
-  const size_t fsz = (size_t)TL * FSP;
-  const size_t sm = sizeof(long long) * 2 * TL + sizeof(T) * (((size_t)lay.total() + 1) & ~(size_t)1) +
-                    sizeof(T) * (nbuf + 1) * fsz + 64;
-  if (sm > 225 * 1024) return out;
-  const int by_smem = (int)((228 * 1024) / (sm + 1024));
-  const int by_regs = 65536 / (regs * threads);
-  const int per_sm = std::max(1, std::min(std::min(by_smem, by_regs), 16));
-  const int64_t tiles = (n_lines + TL - 1) / TL;
-  const int64_t grid = std::min<int64_t>(tiles, (int64_t)nsm * per_sm);
-  out = {TL, 0, FSP, nbuf, (int)grid, sm};
-  return out;
-}
-
-// many lines (3-D grids) and long enough lines: the lane-per-line kernel
-bool use_lane_kernel(const tpf_ccd_plan* p, int64_t n_lines, bool periodic, bool contig) {
-  if (p->n_rows < 128 || p->n_rows > 2048) return false;
-  if (periodic != (p->bc == TPF_BC_PERIODIC)) return false;   // closure overrides on a periodic plan
-  return n_lines >= 148LL * 4 * 32;
-}
-
-// Launch shape of the lane kernel: warps per block, f-tile ring depth, cap on
-// resident blocks per SM.  Every shape computes each line with the same
-// arithmetic, so the results are bitwise identical; only the speed differs.
-using LaneShape = LaneShape_;
-
-template <typename T>
-using LaneFn = void (*)(CcdArgs, const T*, int);
-
-template <typename T, int NB>
-LaneFn<T> lane_fn_nb(bool periodic, bool plain, bool contig) {
-  if (contig)
-    return periodic ? ccd_lane_kernel<T, true, false, NB, true> : ccd_lane_kernel<T, false, false, NB, true>;
-  if (periodic) return plain ? ccd_lane_kernel<T, true, true, NB, false> : ccd_lane_kernel<T, true, false, NB, false>;
-  return plain ? ccd_lane_kernel<T, false, true, NB, false> : ccd_lane_kernel<T, false, false, NB, false>;
-}
-
-template <typename T>
-int run_lane(const tpf_ccd_plan* p, const CcdArgs& a, bool periodic, bool contig, const LaneShape& sh,
-             cudaStream_t stream) {
-  const int W = sh.warps;
-  const int P = (p->n_rows + kLaneCR - 1) / kLaneCR;
-  const size_t per_warp = (size_t)(sh.nbuf + (contig ? 1 : 0)) * (kLaneCR + 2) * (contig ? 33 : 32) + 64 * (size_t)P;
-  const size_t smem = sizeof(T) * ((((size_t)p->ltab_total + 1) & ~(size_t)1) + W * per_warp);
-  TPF_CHECK_ARG(smem <= 225 * 1024, "CCD lane kernel: axis of %lld points needs too much shared memory",
-                (long long)p->n_pts);
-  const bool plain = a.d1 && a.d2 && !a.vd_out && !a.J;
-  LaneFn<T> kern = sh.nbuf == 2 ? lane_fn_nb<T, 2>(periodic, plain, contig) : lane_fn_nb<T, 3>(periodic, plain, contig);
-  TPF_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  int per_sm = 0;
-  TPF_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * W, smem));
-  per_sm = std::max(1, std::min(per_sm, sh.max_bps));
-  const int64_t groups = (a.n_lines + 31) / 32;
-  const int64_t blocks = std::min<int64_t>((groups + W - 1) / W, (int64_t)tpf::sm_count() * per_sm);
-  const T* lt = std::is_same<T, double>::value ? reinterpret_cast<const T*>(p->d_ltab)
-                                               : reinterpret_cast<const T*>(p->d_ltabf);
-  kern<<<(unsigned)blocks, 32 * W, smem, stream>>>(a, lt, p->ltab_total);
+  const bool plain = !a.J && !a.vd_out && !a.cr_out;
+  if (contig) {
+    // 16-byte pieces where the pitch is n and every block's run of every array starts on 16 bytes
+    const bool vec = sh.pitch == p->n_pts && ((size_t)sh.TL * p->n_pts * sizeof(T)) % 16 == 0 &&
+                     (((uintptr_t)a.f | (uintptr_t)a.d1 | (uintptr_t)a.d2) & 15) == 0;
+    auto pick = [&](auto pl) {
+      constexpr bool PL = decltype(pl)::value;
+      return per ? ccd_chunk_contig_kernel<T, kChunkR, true, PL> : ccd_chunk_contig_kernel<T, kChunkR, false, PL>;
+    };
+    auto kern = plain ? pick(std::true_type{}) : pick(std::false_type{});
+    TPF_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    kern<<<sh.blocks, sh.threads, sh.smem, s>>>(a, *K, g, Q, sh.pitch, vec ? 1 : 0);
+  } else {
+    auto pick = [&](auto epi, auto st) {
+      constexpr int E = decltype(epi)::value;
+      constexpr bool S = decltype(st)::value;
+      return per ? ccd_chunk_strided_kernel<T, kChunkR, true, E, S> : ccd_chunk_strided_kernel<T, kChunkR, false, E, S>;
+    };
+    auto pick2 = [&](auto epi) { return sh.staged ? pick(epi, std::true_type{}) : pick(epi, std::false_type{}); };
+    auto kern = a.cr_out   ? pick2(std::integral_constant<int, kChunkCorrector>{})
+                : a.vd_out ? pick2(std::integral_constant<int, kChunkVd>{})
+                : a.J      ? pick2(std::integral_constant<int, kChunkMetric>{})
+                           : pick2(std::integral_constant<int, kChunkPlain>{});
+    if (sh.staged) TPF_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    kern<<<sh.blocks, sh.threads, sh.smem, s>>>(a, *K, g, Q);
+  }
   TPF_CUDA_TRY(cudaGetLastError());
-  return TPF_OK;
-}
-
-// Autotuner: on the first call of a (lines, axis kind, boundary, epilogue,
-// dtype) combination, time the candidate shapes with CUDA events (one warm-up
-// and two timed launches each) and keep the fastest in the plan.  Skipped while
-// the stream is being captured into a graph (the default shape runs).
-template <typename T>
-int launch_lane(const tpf_ccd_plan* p, const CcdArgs& a, bool periodic, bool contig, cudaStream_t stream) {
-  const bool plain = a.d1 && a.d2 && !a.vd_out && !a.J;
-  const uint64_t key = ((uint64_t)a.n_lines << 8) | ((uint64_t)contig << 0) | ((uint64_t)periodic << 1) |
-                       ((uint64_t)plain << 2) | ((uint64_t)(sizeof(T) == 8) << 3);
-  auto it = p->lane_tuned.find(key);
-  if (it != p->lane_tuned.end()) return run_lane<T>(p, a, periodic, contig, it->second, stream);
-  const LaneShape def{4, std::is_same<T, double>::value ? 3 : 2, 64};
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  TPF_CUDA_TRY(cudaStreamIsCapturing(stream, &cs));
-  // an accumulating (or in-place) epilogue must run exactly once: no tuning runs for it
-  if (!p->autotune || cs != cudaStreamCaptureStatusNone || (a.vd_out && a.vd_accumulate) ||
-      (a.cr_out && a.cr_out == a.cr_u))
-    return run_lane<T>(p, a, periodic, contig, def, stream);
-  const LaneShape cand[] = {{4, 3, 64}, {4, 2, 64}, {4, 3, 2}, {4, 2, 3}, {2, 3, 64}, {2, 2, 64}, {4, 2, 2}};
-  cudaEvent_t e0, e1;
-  TPF_CUDA_TRY(cudaEventCreate(&e0));
-  TPF_CUDA_TRY(cudaEventCreate(&e1));
-  float best = 1e30f;
-  LaneShape bs = def;
-  int st = TPF_OK;
-  for (const LaneShape& c : cand) {
-    if ((st = run_lane<T>(p, a, periodic, contig, c, stream))) {
-      if (st != TPF_EINVAL) break;
-      st = TPF_OK;   // a shape that does not fit in shared memory is skipped
-      continue;
-    }
-    cudaEventRecord(e0, stream);
-    for (int r = 0; r < 2 && !st; ++r) st = run_lane<T>(p, a, periodic, contig, c, stream);
-    cudaEventRecord(e1, stream);
-    if (cudaEventSynchronize(e1) != cudaSuccess || st) break;
-    float ms = 0.f;
-    cudaEventElapsedTime(&ms, e0, e1);
-    if (ms < best) {
-      best = ms;
-      bs = c;
-    }
-  }
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
-  if (st) return st;
-  p->lane_tuned[key] = bs;
-  // the results of the last candidate are already in place and identical for every shape
   return TPF_OK;
 }
 
@@ -1971,20 +986,10 @@ int launch_ccd(const tpf_ccd_plan* p, int64_t outer, int64_t inner, const void* 
   TPF_CHECK_ARG(!corrector || (f != corrector->cr_out && f != corrector->cr_u && f != corrector->cr_rho),
                 "the pressure must not alias the velocity or density arrays");
   TPF_CHECK_ARG(n_lines < ((int64_t)1 << 31), "too many lines");
-  // warp kernel: chunks of 8 rows, 1, 2 or 4 warps per line (lines up to 1024 rows)
-  const bool warp = p->C == 8 && p->n_rows <= 32 * 8 * 4;
-  const int W = p->n_rows <= 256 ? 1 : (p->n_rows <= 512 ? 2 : 4);
-  LaunchShape s = !warp ? pick_shape<T>(p, contig, n_lines) : pick_warp_shape<T, 8>(p, n_lines, W);
-  TPF_CHECK_ARG(s.TL > 0, "CCD axis of %lld points does not fit the line kernel's shared memory",
-                (long long)p->n_pts);
   CcdArgs a{};
   a.f = f; a.d1 = d1; a.d2 = d2;
   a.outer = outer; a.inner = inner; a.n_lines = n_lines;
-  a.n = (int)p->n_pts; a.n_rows = p->n_rows; a.C = p->C; a.P = p->P; a.H0 = p->H0; a.TL = s.TL;
-  a.tl_shift = 0;
-  while ((1 << a.tl_shift) < s.TL) ++a.tl_shift;
-  a.LS = s.LS; a.FS = (contig || warp) ? s.FS : 0; a.nbuf = s.nbuf;
-  a.n_tiles = (int)((n_lines + s.TL - 1) / s.TL);
+  a.n = (int)p->n_pts; a.n_rows = p->n_rows; a.C = p->C; a.P = p->P; a.H0 = p->H0;
   a.tab_total = TabLayout{p->C, p->H0}.total();
   a.tab = p->d_tab;
   a.tabT = std::is_same<T, double>::value ? (const void*)p->d_tab : (const void*)p->d_tabf;
@@ -2005,81 +1010,25 @@ int launch_ccd(const tpf_ccd_plan* p, int64_t outer, int64_t inner, const void* 
     a.cr_wall = corrector->cr_wall;
   }
   const bool per = (p->bc == TPF_BC_PERIODIC) && !a.ovl && !a.ovr;
-  if (use_lane_kernel(p, n_lines, per, contig)) return launch_lane<T>(p, a, per, contig, stream);
+  if (per == (p->bc == TPF_BC_PERIODIC)) {
+    const ChunkShape sh = chunk_shape<T>(p, contig, n_lines, inner);
+    if (sh.TL > 0) return launch_chunk<T>(p, a, per, contig, sh, stream);
+  }
+  // longer lines, and closure overrides on a periodic plan
+  const LaunchShape s = pick_shape<T>(p, contig, n_lines);
+  TPF_CHECK_ARG(s.TL > 0, "CCD axis of %lld points does not fit the line kernel's shared memory",
+                (long long)p->n_pts);
+  a.TL = s.TL;
+  a.tl_shift = 0;
+  while ((1 << a.tl_shift) < s.TL) ++a.tl_shift;
+  a.LS = s.LS; a.FS = contig ? s.FS : 0; a.nbuf = s.nbuf;
+  a.n_tiles = (int)((n_lines + s.TL - 1) / s.TL);
   void (*kern)(CcdArgs);
-  if (!warp) {
-    if (per) kern = contig ? ccd_line_kernel<T, true, true> : ccd_line_kernel<T, true, false>;
-    else kern = contig ? ccd_line_kernel<T, false, true> : ccd_line_kernel<T, false, false>;
-  } else {
-#define TPF_WARP_KERN(WW)                                                                               \
-  if (per) kern = contig ? ccd_warp_kernel<T, true, true, 8, WW> : ccd_warp_kernel<T, true, false, 8, WW>; \
-  else kern = contig ? ccd_warp_kernel<T, false, true, 8, WW> : ccd_warp_kernel<T, false, false, 8, WW>;
-    if (W == 1) { TPF_WARP_KERN(1) }
-    else if (W == 2) { TPF_WARP_KERN(2) }
-    else { TPF_WARP_KERN(4) }
-#undef TPF_WARP_KERN
-  }
-  auto launch = [&](const LaunchShape& sh) -> int {
-    CcdArgs b = a;
-    b.TL = sh.TL;
-    b.tl_shift = 0;
-    while ((1 << b.tl_shift) < sh.TL) ++b.tl_shift;
-    b.FS = (contig || warp) ? sh.FS : 0;
-    b.LS = sh.LS;
-    b.nbuf = sh.nbuf;
-    b.n_tiles = (int)((n_lines + sh.TL - 1) / sh.TL);
-    TPF_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem));
-    kern<<<sh.grid, warp ? 32 * W * sh.TL : sh.TL * p->P, sh.smem, stream>>>(b);
-    TPF_CUDA_TRY(cudaGetLastError());
-    return TPF_OK;
-  };
-  if (!warp) return launch(s);
-  // Warp kernel: the launch shape (lines per block, tile buffers) is picked by
-  // timing on the first call of each (line count, axis kind, boundary,
-  // outputs, dtype) combination, like the lane kernel's; every shape gives
-  // identical results (the lines are solved independently).
-  const bool plain = a.d1 && a.d2 && !a.vd_out && !a.J && !a.cr_out;
-  const uint64_t key = ((uint64_t)n_lines << 8) | (1ull << 7) | ((uint64_t)contig << 0) | ((uint64_t)per << 1) |
-                       ((uint64_t)plain << 2) | ((uint64_t)(sizeof(T) == 8) << 3) | ((uint64_t)W << 4);
-  auto it = p->lane_tuned.find(key);
-  if (it != p->lane_tuned.end()) {
-    const LaunchShape ts = warp_shape<T, 8>(p, n_lines, W, it->second.warps, it->second.nbuf);
-    if (ts.TL > 0) return launch(ts);
-  }
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  TPF_CUDA_TRY(cudaStreamIsCapturing(stream, &cs));
-  if (!p->autotune || cs != cudaStreamCaptureStatusNone || (a.vd_out && a.vd_accumulate) ||
-      (a.cr_out && a.cr_out == a.cr_u))
-    return launch(s);
-  cudaEvent_t e0, e1;
-  TPF_CUDA_TRY(cudaEventCreate(&e0));
-  TPF_CUDA_TRY(cudaEventCreate(&e1));
-  float best = 1e30f;
-  LaunchShape bs = s;
-  int st = TPF_OK;
-  const int tls[4] = {8, 4, 2, 1};
-  for (int ti = 0; ti < 4 && !st; ++ti) {
-    for (int nbuf = 1; nbuf <= 2 && !st; ++nbuf) {
-      const LaunchShape c = warp_shape<T, 8>(p, n_lines, W, tls[ti], nbuf);
-      if (c.TL == 0) continue;
-      if ((st = launch(c))) break;
-      cudaEventRecord(e0, stream);
-      for (int r = 0; r < 2 && !st; ++r) st = launch(c);
-      cudaEventRecord(e1, stream);
-      if (cudaEventSynchronize(e1) != cudaSuccess || st) break;
-      float ms = 0.f;
-      cudaEventElapsedTime(&ms, e0, e1);
-      if (ms < best) {
-        best = ms;
-        bs = c;
-      }
-    }
-  }
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
-  if (st) return st;
-  p->lane_tuned[key] = LaneShape_{bs.TL, bs.nbuf, 0};
-  // the last candidate's results are in place and identical for every shape
+  if (per) kern = contig ? ccd_line_kernel<T, true, true> : ccd_line_kernel<T, true, false>;
+  else kern = contig ? ccd_line_kernel<T, false, true> : ccd_line_kernel<T, false, false>;
+  TPF_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem));
+  kern<<<s.grid, s.TL * p->P, s.smem, stream>>>(a);
+  TPF_CUDA_TRY(cudaGetLastError());
   return TPF_OK;
 }
 
@@ -2298,18 +1247,19 @@ int tpf_ccd_plan_create(tpf_ccd_plan** out, int64_t n_pts, double h, int bc, int
     return TPF_ECUDA;
   }
   {
-    const std::vector<double>& lt = p->ltab_host;
-    std::vector<float> ltf(lt.begin(), lt.end());
-    p->ltab_total = (int)lt.size();
-    if (cudaMalloc(&p->d_ltab, lt.size() * sizeof(double)) != cudaSuccess ||
-        cudaMalloc(&p->d_ltabf, lt.size() * sizeof(float)) != cudaSuccess ||
-        cudaMemcpy(p->d_ltab, lt.data(), lt.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(p->d_ltabf, ltf.data(), ltf.size() * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess) {
-      tpf::set_error("allocation / copy of the CCD lane table failed");
+    std::vector<double> G;
+    p->c64 = chunk_tables<kChunkR>(p, G);
+    p->c32 = cast_chunk<float>(p->c64);
+    const std::vector<float> Gf(G.begin(), G.end());
+    if (cudaMalloc(&p->d_g64, G.size() * sizeof(double)) != cudaSuccess ||
+        cudaMalloc(&p->d_g32, G.size() * sizeof(float)) != cudaSuccess ||
+        cudaMemcpy(p->d_g64, G.data(), G.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaMemcpy(p->d_g32, Gf.data(), Gf.size() * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess) {
+      tpf::set_error("allocation / copy of the CCD wall table failed");
       cudaFree(p->d_tab);
       cudaFree(p->d_tabf);
-      cudaFree(p->d_ltab);
-      cudaFree(p->d_ltabf);
+      cudaFree(p->d_g64);
+      cudaFree(p->d_g32);
       delete p;
       return TPF_ECUDA;
     }
@@ -2320,8 +1270,7 @@ int tpf_ccd_plan_create(tpf_ccd_plan** out, int64_t n_pts, double h, int bc, int
 
 int tpf_ccd_plan_set_autotune(tpf_ccd_plan* p, int enable) {
   TPF_CHECK_ARG(p != nullptr, "plan is NULL");
-  p->autotune = enable != 0;
-  if (!enable) p->lane_tuned.clear();
+  (void)enable;   // launch shapes follow from the sizes
   return TPF_OK;
 }
 
@@ -2329,8 +1278,8 @@ int tpf_ccd_plan_destroy(tpf_ccd_plan* p) {
   if (!p) return TPF_OK;
   cudaFree(p->d_tab);
   cudaFree(p->d_tabf);
-  cudaFree(p->d_ltab);
-  cudaFree(p->d_ltabf);
+  cudaFree(p->d_g64);
+  cudaFree(p->d_g32);
   cudaFree(p->d_J);
   cudaFree(p->d_rfac);
   delete p;
