@@ -32,6 +32,7 @@
 #include <mutex>
 #include <memory>
 #include <numeric>
+#include <type_traits>
 #include <vector>
 
 namespace {
@@ -2088,6 +2089,8 @@ __global__ void cgs_finish_kernel(int ndof, int pin, const CgScal* sc, const dou
 
 // ---- handle -------------------------------------------------------------------------
 
+#include "gmres_grid.cuh"
+
 struct tpf_ppe {
   int ndim = 2;
   Grid3 g{};
@@ -2137,6 +2140,9 @@ struct tpf_ppe {
   size_t band_pub_len = 0;
   FlagSlot* band_slots = nullptr; // sums and halo rows of the FP64 band-resident PCG
   size_t band_slots_len = 0;
+  FlagSlot* gg_slots = nullptr;   // exchange slots of the one-launch GMRES
+  size_t gg_slots_len = 0;
+  GmresGridOut* gg_out = nullptr;
   int cg_kernel = 0;              // 0 auto, 1 global-memory persistent PCG, 2 band-resident PCG
   SolveStatus* st = nullptr;
   int coop_blocks = 0;
@@ -2185,6 +2191,18 @@ LineArgs line_args(const Grid3& g, int axis) {
     L.lines = g.n0 * g.n1; L.n = g.n2; L.stride = 1; L.lmod = 1 << 30; L.lstride_hi = 0; L.lstride_lo = g.n2;
   }
   return L;
+}
+
+// dynamic shared memory a persistent kernel may use: the opt-in limit less its static scratch
+bool smem_optin(size_t* limit) {
+  int dev = 0, optin = 0;
+  cudaGetDevice(&dev);
+  if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  *limit = (size_t)optin - 4096;
+  return true;
 }
 
 int ensure_gmres(tpf_ppe* h) {
@@ -2284,6 +2302,116 @@ int precond_L(tpf_ppe* h, const double* r, double* z, cudaStream_t s, const int*
   return TPF_OK;
 }
 
+// ---- one-launch GMRES (gmres_grid.cuh) -------------------------------------------
+struct GmresGridPlan {
+  int rows, G, m, k, ld;
+  bool vs;
+  size_t smem;
+};
+// Applies to 2-D systems whose lines fit a warp (544 nodes) and whose rows,
+// line factors and Hessenberg matrix fit the shared memory of one SM per
+// block; a block has up to a node per thread in whole rows, or what 148 blocks
+// need.  Up to that limit it is the faster side throughout (33^2: 14 us a column
+// against 57 as kernels, 129 x 97: 13 against 65, 201^2: 23 against 81); at
+// 513^2 the line factors of a block no longer fit and the kernels run (190 us).
+bool gmres_grid_plan(const tpf_ppe* h, GmresGridPlan& P) {
+  const Grid3& g = h->g;
+  if (h->ndim != 2 || g.N2 != 0 || h->o.precond == TPF_PRECOND_LINE_PCR) return false;
+  const int need = (std::max(g.n0, g.n1) + 31) / 32;
+  P.k = 0;
+  for (int k : kGgLane)
+    if (k >= need) { P.k = k; break; }
+  if (!P.k) return false;
+  const int most = std::min(kGgMaxGrid, tpf::sm_count());
+  P.rows = std::max((g.n0 + most - 1) / most, std::max(1, kGgThreads / g.n1));
+  P.rows = std::min(P.rows, g.n0);
+  P.G = (g.n0 + P.rows - 1) / P.rows;
+  P.m = std::min(h->o.restart, g.ndof);
+  P.ld = (P.m + 2 + 7) / 8 * 8;
+  size_t limit = 0;
+  if (!smem_optin(&limit)) return false;
+  const size_t rest = gg_smem_doubles(g.n0, g.n1, P.rows, P.G, P.m, h->o.precond == TPF_PRECOND_LINE);
+  const size_t basis = (size_t)P.rows * g.n1 * P.m;
+  P.vs = sizeof(double) * (rest + basis) <= limit;
+  P.smem = sizeof(double) * (rest + (P.vs ? basis : 0));
+  return P.smem <= limit;
+}
+
+int solve_gmres_grid(tpf_ppe* h, const GmresGridPlan& P, const double* rhs, double* p, const double* p_init,
+                     cudaStream_t s, tpf_ppe_result* res) {
+  const Grid3& g = h->g;
+  const int n = g.ndof;
+  int st;
+  if (!P.vs && (st = ensure_gmres(h))) return st;
+  const size_t edges = (size_t)2 * P.G * 2 * g.n1, dots = (size_t)2 * P.G * P.ld, slots = 4 * (size_t)n + edges + dots;
+  if (h->gg_slots_len < slots) {
+    if ((st = dalloc(h, &h->gg_slots, slots))) return st;
+    h->gg_slots_len = slots;
+  }
+  if (!h->gg_out && (st = dalloc(h, &h->gg_out, 1))) return st;
+  copy_pin0_kernel<<<ew_grid(h), 256, 0, s>>>(n, g.pin, rhs, h->b);
+  if (p_init) copy_pin0_kernel<<<ew_grid(h), 256, 0, s>>>(n, g.pin, p_init, h->x);
+  else TPF_CUDA_TRY(cudaMemsetAsync(h->x, 0, sizeof(double) * n, s));
+  TPF_CUDA_TRY(cudaMemsetAsync(h->gg_slots, 0, sizeof(FlagSlot) * slots, s));   // epochs start at 1
+  TPF_CUDA_TRY(cudaMemsetAsync(h->err, 0, sizeof(int), s));
+  GmresGridArgs a{};
+  a.g = g;
+  a.geo = Geo{{h->dv[0], h->dv[1], h->dv[2]}, {h->dface[0], h->dface[1], h->dface[2]}};
+  a.s0 = h->s[0];
+  a.s1 = h->s[1];
+  for (int ax = 0; ax < 2; ++ax) {
+    a.lo[ax] = h->tlo[ax];
+    a.den[ax] = h->tden[ax];
+    a.cp[ax] = h->tcp[ax];
+  }
+  a.dinvL = h->dinvL;
+  a.precond = h->o.precond;
+  a.b = h->b;
+  a.x = h->x;
+  a.V = h->V;
+  a.wt = h->gg_slots;
+  a.zt = a.wt + 2 * (size_t)n;
+  a.edges = a.zt + 2 * (size_t)n;
+  a.dots = a.edges + edges;
+  a.ld = P.ld;
+  a.err = h->err;
+  a.out = h->gg_out;
+  a.tol = h->o.tol;
+  a.maxiter = h->o.maxiter;
+  a.m = P.m;
+  a.rows = P.rows;
+  a.k = P.k;
+  a.x_nonzero = p_init ? 1 : 0;
+  void* fn = P.vs ? (void*)gmres_grid_kernel<true> : (void*)gmres_grid_kernel<false>;
+  size_t limit = P.smem;
+  smem_optin(&limit);
+  TPF_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit));
+  void* args[] = {&a};
+  TPF_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(P.G), dim3(kGgThreads), args, P.smem, s));
+  copy_pin0_kernel<<<ew_grid(h), 256, 0, s>>>(n, g.pin, h->x, p);
+  TPF_CUDA_TRY(cudaGetLastError());
+  GmresGridOut o{};
+  int herr = 0;
+  TPF_CUDA_TRY(cudaMemcpyAsync(&o, h->gg_out, sizeof(o), cudaMemcpyDeviceToHost, s));
+  TPF_CUDA_TRY(cudaMemcpyAsync(&herr, h->err, sizeof(int), cudaMemcpyDeviceToHost, s));
+  TPF_CUDA_TRY(cudaStreamSynchronize(s));
+  if (herr) {
+    tpf::set_error("GMRES exchange timed out; the solve was aborted");
+    return TPF_EABORT;
+  }
+  res->refinements = 0;
+  res->iterations = o.inner;
+  res->applies = o.applies;
+  res->rel_residual = o.bnrm2 > 0.0 ? o.rnorm / o.bnrm2 : 0.0;
+  res->info = o.converged ? 0 : (int)std::min<long long>(h->o.maxiter, 0x7fffffff);
+  if (!o.converged) {
+    tpf::set_error("PPESolverFVMMatrixFree did not converge cleanly (info=%d); no alternate PPE solver was applied.",
+                   res->info);
+    return TPF_ENOCONV;
+  }
+  return TPF_OK;
+}
+
 // SciPy 1.18.1 gmres restated on the device (gmres.cuh) over the FVM
 // operator and the handle's preconditioner.
 int solve_gmres(tpf_ppe* h, const double* rhs, double* p, const double* p_init, cudaStream_t s,
@@ -2296,6 +2424,8 @@ int solve_gmres(tpf_ppe* h, const double* rhs, double* p, const double* p_init, 
   TPF_CHECK_ARG(cap_state == cudaStreamCaptureStatusNone,
                 "the GMRES route reads its residual on the host between restart cycles and cannot be captured "
                 "into a CUDA graph (the CG route can)");
+  GmresGridPlan gp;
+  if (gmres_grid_plan(h, gp)) return solve_gmres_grid(h, gp, rhs, p, p_init, s, res);
   if ((st = ensure_gmres(h))) return st;
   GmresWork W;
   W.n = n;
@@ -2368,17 +2498,6 @@ struct BandPlan {
   size_t smem;
   bool mixed;
 };
-// dynamic shared memory a band kernel may use: the opt-in limit less its static scratch
-bool band_smem_limit(size_t* limit) {
-  int dev = 0, optin = 0;
-  cudaGetDevice(&dev);
-  if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
-  *limit = (size_t)optin - 4096;
-  return true;
-}
 // most blocks a system is spread over: one per SM, none shorter than a grid
 // row; in FP64 down to one node per thread (64^2: 2.11 us an iteration on 17
 // blocks, 2.35 on 9, 2.48 on 34; 130^2: 2.27 on 68, 2.51 on 34)
@@ -2394,7 +2513,7 @@ bool band_plan(const tpf_ppe* h, BandPlan& bp, bool mixed) {
   if (g.n1 > kBandMaxW) return false;
   const int grid = band_max_grid(h, mixed);
   size_t limit = 0;
-  if (grid < 1 || !band_smem_limit(&limit)) return false;
+  if (grid < 1 || !smem_optin(&limit)) return false;
   bp.grid = grid;
   bp.n_max = (g.ndof + grid - 1) / grid;
   bp.smem = band_smem(bp.n_max, g.n1, mixed, limit);
@@ -2457,7 +2576,7 @@ int launch_band(tpf_ppe* h, const BandPlan& bp, const Cg1Args& c, cudaStream_t s
     TPF_CUDA_TRY(cudaMemsetAsync(h->band_slots, 0, sizeof(FlagSlot) * band_slot_count(h, bp.grid), s));
   void* fn = band_kernel(bp.n_max, bp.mixed, false);
   size_t limit = 0;
-  if (band_smem_limit(&limit))   // always the same value: other threads may launch the same kernel
+  if (smem_optin(&limit))   // always the same value: other threads may launch the same kernel
     TPF_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit));
   void* args[] = {&a};
   TPF_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(bp.grid), dim3(bp.mixed ? kThreads : kBandThreads), args, bp.smem, s));
@@ -3013,7 +3132,7 @@ namespace {
 bool band_batch_plan(tpf_ppe* const* hs, int n, bool mixed, std::vector<int>& nb, std::vector<int>& nmax,
                      size_t& smem) {
   size_t limit = 0;
-  if (!band_smem_limit(&limit)) return false;
+  if (!smem_optin(&limit)) return false;
   const int cap = tpf::sm_count();
   std::vector<int> lo(n), hi(n);
   double wsum = 0.0;
@@ -3254,7 +3373,7 @@ int solve_band_batch(tpf_ppe* const* hs, int n, const double* const* rhs, const 
   }
   void* fn = band_kernel(*std::max_element(nmax.begin(), nmax.end()), mixed, true);
   size_t limit = smem;
-  band_smem_limit(&limit);
+  smem_optin(&limit);
   TPF_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit));
   band_setup_kernel<<<u->first[n], 256, 0, s>>>(*u);
   void* args[] = {b.get()};
