@@ -2090,6 +2090,7 @@ __global__ void cgs_finish_kernel(int ndof, int pin, const CgScal* sc, const dou
 // ---- handle -------------------------------------------------------------------------
 
 #include "gmres_grid.cuh"
+#include "march_pcg.cuh"
 
 struct tpf_ppe {
   int ndim = 2;
@@ -2133,6 +2134,7 @@ struct tpf_ppe {
   BandOutcome* batch_out = nullptr;    // per system: status of a band-resident batch
   int batch_out_len = 0;
   int* batch_pending = nullptr;        // systems still iterating in a batched streaming solve
+  FlagSlot* march_slots = nullptr;     // sums of the marching PCG
   int pending = 0;                     // captured CG solve: 1 status in st, 2 in cgs
   cudaStream_t cap = nullptr;          // stream the cycle is captured on (never the caller's)
   long long gm_key[6] = {};
@@ -2583,7 +2585,69 @@ int launch_band(tpf_ppe* h, const BandPlan& bp, const Cg1Args& c, cudaStream_t s
   return TPF_OK;
 }
 
-// Streaming PCG: the iteration as two kernels at full occupancy, chunks of
+// ---- marching PCG (march_pcg.cuh) -------------------------------------------------
+// Applies where a plane's row of axis 2 is short enough that three stages fit
+// the shared memory of an SM (n2 up to about 900); beyond that the two streaming
+// kernels run.  Where both can, this is the faster one (streaming kernels ->
+// here, us an iteration): 25^3 9.5 -> 7.5, 65^3 18.4 -> 11.0, 97^3 27.5 -> 19.9,
+// 129^3 66.3 -> 43.9, 1025^2 29.2 -> 25.0.
+bool march_plan(const tpf_ppe* h, MarchArgs& a, int& grid, size_t& smem) {
+  const Grid3& g = h->g;
+  size_t limit = 0;
+  if (!smem_optin(&limit)) return false;
+  limit -= 8192;   // the kernel's static share
+  a.tiles = (g.st0 + kMarchT - 1) / kMarchT;
+  a.T = march_even((g.st0 + a.tiles - 1) / a.tiles);
+  a.units = a.tiles * g.n0;
+  grid = std::min({a.units, tpf::sm_count(), kMarchGrid});
+  a.most = (a.units + grid - 1) / grid;
+  const MarchStage L(a.T, g.n2);
+  const size_t planes = 2 * (size_t)march_even(a.T + 2 * g.n2), w = (size_t)a.most * a.T;
+  auto bytes = [&](int stages, size_t more) { return sizeof(double) * (stages * (size_t)L.size + planes + more); };
+  // w stays on chip where it fits beside the stages, which then need no more
+  // than three (65^3: 10.9 us an iteration with 3 stages, 11.2 with 6); else more
+  // stages are worth more than w (129^3: 43.8 us with 6, 45.0 with 3 and w)
+  a.w_on_chip = bytes(4, w) <= limit;
+  a.stages = 3;
+  while (!a.w_on_chip && a.stages < kMarchStages && bytes(a.stages + 1, 0) <= limit) ++a.stages;
+  smem = bytes(a.stages, a.w_on_chip ? w : 0);
+  return smem <= limit;
+}
+
+int launch_march(tpf_ppe* h, MarchArgs& a, int grid, size_t smem, const Cg1Args& c, cudaStream_t s) {
+  int st;
+  const size_t slots = (size_t)2 * kMarchGrid * kBandLine;
+  if (!h->march_slots && (st = dalloc(h, &h->march_slots, slots))) return st;
+  a.g = c.g;
+  a.s0 = c.s64[0];
+  a.s1 = c.s64[1];
+  a.s2 = c.s64[2];
+  a.dinv = c.v64.dinv;
+  a.b = c.b;
+  a.x = c.x;
+  a.r = h->c64[0];
+  a.z = h->c64[1];
+  a.w = h->c64[2];
+  a.p[0] = h->c64[4];
+  a.p[1] = h->c64[6];
+  a.slots = h->march_slots;
+  a.err = c.err;
+  a.st = c.st;
+  a.tol = c.tol;
+  a.maxiter = c.maxiter;
+  a.x_nonzero = c.x_nonzero;
+  TPF_CUDA_TRY(cudaMemsetAsync(h->march_slots, 0, sizeof(FlagSlot) * slots, s));   // epochs start at 1
+  void* fn = c.g.N2 > 0 ? (void*)march_pcg_kernel<true> : (void*)march_pcg_kernel<false>;
+  size_t limit = 0;
+  if (smem_optin(&limit))   // always the same value: other threads may launch the same kernel
+    TPF_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(limit - 8192)));
+  void* args[] = {&a};
+  TPF_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kMarchT), args, smem, s));
+  return TPF_OK;
+}
+
+// Streaming PCG, where the marching one does not apply: the iteration as two
+// kernels at full occupancy, chunks of
 // kCgsChunk iterations replayed from a CUDA graph (see the kernels above).
 constexpr int kCgsChunk = 32;
 
@@ -2796,9 +2860,14 @@ int solve_cg(tpf_ppe* h, const double* rhs, double* p, const double* p_init, cud
   const bool mixed = (h->o.precision == TPF_PREC_MIXED);
   BandPlan bp;
   const bool band = band_plan(h, bp, mixed);
-  if (!mixed && (h->cg_kernel == 3 || (h->cg_kernel == 0 && !band)))
-    return solve_cg_stream(h, rhs, p, p_init, s, res);
-  if (band) {
+  MarchArgs ma{};
+  int mgrid = 0;
+  size_t msmem = 0;
+  if (!mixed && (h->cg_kernel == 3 || (h->cg_kernel == 0 && !band))) {
+    if (!march_plan(h, ma, mgrid, msmem)) return solve_cg_stream(h, rhs, p, p_init, s, res);
+    int st = launch_march(h, ma, mgrid, msmem, a, s);
+    if (st) return st;
+  } else if (band) {
     int st = launch_band(h, bp, a, s);
     if (st) return st;
   } else {
@@ -2922,7 +2991,7 @@ int tpf_ppe_create(tpf_ppe** out, int ndim, const int64_t* N, const double* cons
   }
   const size_t n = (size_t)ndof;
   for (int a = 0; a < ndim; ++a) {
-    if ((st = dalloc(h, &h->s[a], n))) return fail(st);
+    if ((st = dalloc(h, &h->s[a], n + 1))) return fail(st);   // + 1: march_copy's node of slack, as below
     if ((st = dalloc(h, &h->s32[a], n))) return fail(st);
     if ((st = dalloc(h, &h->tlo[a], n))) return fail(st);
     if ((st = dalloc(h, &h->tden[a], n))) return fail(st);
@@ -2932,12 +3001,12 @@ int tpf_ppe_create(tpf_ppe** out, int ndim, const int64_t* N, const double* cons
   double** d64[] = {&h->dinvS, &h->dinvL, &h->x, &h->r, &h->z, &h->p0, &h->p1, &h->q, &h->b, &h->t1, &h->t2,
                       &h->ones64};
   for (double** pp : d64)
-    if ((st = dalloc(h, pp, n))) return fail(st);
+    if ((st = dalloc(h, pp, n + 1))) return fail(st);
   float** d32[] = {&h->dinvS32, &h->ones32};
   for (float** pp : d32)
     if ((st = dalloc(h, pp, n))) return fail(st);
   for (int k = 0; k < 7; ++k) {
-    if ((st = dalloc(h, &h->c64[k], n))) return fail(st);
+    if ((st = dalloc(h, &h->c64[k], n + 1))) return fail(st);
     if ((st = dalloc(h, &h->c32[k], n))) return fail(st);
   }
   // ones: the identity preconditioner of the CG route ('none')
@@ -2980,6 +3049,7 @@ int tpf_ppe_create(tpf_ppe** out, int ndim, const int64_t* N, const double* cons
       tpf::set_error("cudaStreamCreate failed");
       return fail(TPF_ECUDA);
     }
+    if ((st = dalloc(h, &h->march_slots, (size_t)2 * kMarchGrid * kBandLine))) return fail(st);
   }
   *out = h;
   return TPF_OK;
