@@ -273,5 +273,8 @@ def dptr(t) -> C.c_void_p:
 
 
 def current_stream_handle():
+    """The current device's current stream.  The raw query rather than
+    ``torch.cuda.current_stream().cuda_stream``, which builds a Stream object:
+    0.5 us against 3.5 us of a small operator's 17 us call."""
     import torch
-    return C.c_void_p(int(torch.cuda.current_stream().cuda_stream))
+    return C.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))

@@ -34,13 +34,16 @@ class DeviceView:
 
 
 def to_device(data, dtype=None, device=None) -> DeviceView:
+    import torch
+    if isinstance(data, torch.Tensor) and data.is_cuda:   # first: small operators' calls are bound by the host
+        if dtype is not None and data.dtype != dtype:
+            data = data.to(dtype)
+        return DeviceView(data if data.is_contiguous() else data.contiguous(), False)
     torch = _torch()
     dev = device if device is not None else torch.device("cuda", torch.cuda.current_device())
     if isinstance(data, torch.Tensor):
-        t = data
-        host = not t.is_cuda
-        if host:
-            t = t.pin_memory().to(dev, non_blocking=True) if t.device.type == "cpu" else t.to(dev)
+        t = data.pin_memory().to(dev, non_blocking=True) if data.device.type == "cpu" else data.to(dev)
+        host = True
     elif hasattr(data, "__cuda_array_interface__"):
         t = torch.as_tensor(data, device=dev)
         host = False
