@@ -493,12 +493,13 @@ __global__ void compression_flux_kernel(CompArgs a) {
 // ('periodic': g[n-2] left, g[1] right) or the end node itself ('neumann',
 // 'outflow') (filtered_divergence, reinit_ops.py:83-105; pad_ghost_cells,
 // core/boundary.py:249-292).
+// 193^3 FP64: 39.9 us with a 64-bit division and remainder per node, 33.4 with AxisCoord.
 template <typename T>
-__global__ void filtered_div_kernel(int64_t outer, int64_t n, int64_t inner, int pad, double eps_d, const T* g,
+__global__ void filtered_div_kernel(int64_t tot, tpf::AxisCoord pos, int pad, double eps_d, const T* g,
                                     const double* J, int accumulate, T* div) {
-  const int64_t tot = outer * n * inner;
+  const int64_t n = pos.n, inner = pos.inner;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < tot; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t k = (i / inner) % n;
+    const int64_t k = pos(i);
     const double c = (double)g[i];
     double m, p;
     if (k > 0) m = (double)g[i - inner];
@@ -778,13 +779,14 @@ static int filtered_divergence_axis(int ndim, const int64_t* shape, int axis, in
   const int64_t n = shape[axis];
   TPF_CHECK_ARG(n >= 3, "at least 3 nodes along the axis");
   const int64_t tot = outer * n * inner;
+  const tpf::AxisCoord pos(outer, n, inner);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (dtype == TPF_F64)
-    filtered_div_kernel<double><<<blocks_for(tot, 16), 256, 0, st>>>(outer, n, inner, pad, eps_d,
+    filtered_div_kernel<double><<<blocks_for(tot, 16), 256, 0, st>>>(tot, pos, pad, eps_d,
                                                                     static_cast<const double*>(g), J, accumulate,
                                                                     static_cast<double*>(div));
   else
-    filtered_div_kernel<float><<<blocks_for(tot, 16), 256, 0, st>>>(outer, n, inner, pad, eps_d,
+    filtered_div_kernel<float><<<blocks_for(tot, 16), 256, 0, st>>>(tot, pos, pad, eps_d,
                                                                    static_cast<const float*>(g), J, accumulate,
                                                                    static_cast<float*>(div));
   TPF_CUDA_TRY(cudaGetLastError());

@@ -28,6 +28,7 @@ struct LowArgs {
   double re;
   int64_t outer, n, inner;
   int accumulate, finalize;
+  tpf::AxisCoord pos;
 };
 
 template <typename T>
@@ -46,7 +47,7 @@ __global__ void lowfd_kernel(LowArgs a) {
   const int64_t tot = a.outer * a.n * a.inner;
   const int64_t s = a.inner, n = a.n;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < tot; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t k = (i / s) % n;
+    const int64_t k = a.pos(i);
     double d;
     if (k == 0) {
       d = rn_sub(val<T>(a, i + s), val<T>(a, i)) / a.dx0;
@@ -106,6 +107,7 @@ extern "C" int tpf_visc_lowfd_axis(int ndim, const int64_t* shape, int axis, con
   TPF_CHECK_ARG(A.n >= 3, "at least 3 nodes along the axis");
   const int64_t tot = A.outer * A.n * A.inner;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  A.pos = tpf::AxisCoord(A.outer, A.n, A.inner);
   if (dtype == TPF_F64) lowfd_kernel<double><<<blocks_for(tot), 256, 0, st>>>(A);
   else lowfd_kernel<float><<<blocks_for(tot), 256, 0, st>>>(A);
   TPF_CUDA_TRY(cudaGetLastError());
