@@ -487,8 +487,8 @@ def main(argv=None):
     roof_plain = {"kernel": "cg1_band_kernel", "bound": "hbm", "achieved": round(ach64, 1), "peak": peak,
                   "peak_kind": peak_kind, "unit": "GB/s", "frac": round(ach64 / peak, 3),
                   "traffic": PCG_BAND_DRAM_BYTES_PER_SOLVE,
-                  "note": "112 B/DOF/iteration algorithmic over the solve; vectors live in shared memory, "
-                          "DRAM traffic is the inputs once (ncu); the iteration is bound by the grid reduction"}
+                  "note": "112 B/DOF/iteration algorithmic over the solve; vectors live in registers, "
+                          "DRAM traffic is the inputs once (ncu); the iteration is bound by the exchange between blocks"}
     # the learned solve's top kernel by time share: the blocked damped-Jacobi
     # smoother (48 B per node and launch algorithmic, 4 sweeps per launch)
     from twophaseflow_b200.kernel_cases import smoother_case

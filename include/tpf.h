@@ -447,22 +447,23 @@ int tpf_ppe_set_options(tpf_ppe* h, const tpf_ppe_options* opts);
  *     (any grid, FP64 or mixed);
  * 2 = the band-resident kernel: 2-D systems whose nodes, split into one
  *     contiguous range per SM (at least one row each, at most 768 nodes per
- *     row), fit in shared memory with 12 FP64 vectors (~550^2 on a B200) or,
- *     mixed, 11 FP32 vectors and x in FP64 (~770^2); only the ranges' first
- *     and last rows cross L2 each iteration.
+ *     row), fit the SM's registers in FP64 (2816 nodes per SM, ~640^2 on a
+ *     B200) or, mixed, its shared memory with 11 FP32 vectors and x in FP64
+ *     (~770^2); only the ranges' first and last rows cross L2 each iteration.
  *     TPF_EINVAL from tpf_ppe_solve when it does not apply;
- * 3 = streaming (FP64): each iteration as two ordinary full-occupancy
- *     kernels (vector update; stencil + inner products, the last block
- *     advancing the scalars on the device), chunks of 32 iterations
- *     replayed from a CUDA graph.  The mixed-precision route keeps 1. */
+ * 3 = streaming (FP64): one cooperative launch that marches over the planes
+ *     and streams the vectors from L2 / HBM; where the last axis is too long
+ *     for its shared memory (above ~900 nodes in 3-D), each iteration as two
+ *     ordinary kernels, chunks of 32 iterations replayed from a CUDA graph.
+ *     The mixed-precision route keeps 1. */
 int tpf_ppe_set_cg_kernel(tpf_ppe* h, int kind);
 
 /* Stream capture (no counterpart in the reference, which has no CUDA graphs):
  * tpf_ppe_solve with method TPF_PPE_CG may be called while `stream` is being
  * captured into a CUDA graph.  The whole solve is then recorded in the graph
- * (the persistent kernels as one cooperative launch; the streaming PCG as a
- * conditional WHILE node whose body runs 32 iterations and re-tests the
- * device-side convergence state), nothing is read back, and the result
+ * (the one-launch kernels as one cooperative launch; the two-kernel streaming
+ * PCG as a conditional WHILE node whose body runs 32 iterations and re-tests
+ * the device-side convergence state), nothing is read back, and the result
  * fields are -1.  After a replay, tpf_ppe_read_result synchronizes `stream`
  * and returns that replay's result and status (TPF_ENOCONV as tpf_ppe_solve).
  * The GMRES route reads its residual on the host and returns TPF_EINVAL under
@@ -497,11 +498,10 @@ int tpf_ppe_solve(tpf_ppe* h, const double* rhs, const double* rho, double* p,
 /* Batched solve (no counterpart in the reference, which solves one system
  * per call): n independent systems (n <= 64, each its own handle and grid,
  * all with method TPF_PPE_CG and one precision).  When every system is 2-D
- * and all their bands fit in shared memory at once (the systems' nodes
- * summing to at most ~340 000 in FP64, ~640 000 mixed, on 148 SMs): ONE
- * cooperative launch in which every system runs the band-resident PCG on its
- * own share of the SMs (proportional to ndof^1.5, its expected work) with its
- * own grid barrier.  Otherwise, FP64: the batched streaming PCG -- every
+ * and all their ranges fit on chip at once (the systems' nodes summing to at
+ * most ~400 000 in FP64, ~640 000 mixed, on 148 SMs): ONE cooperative launch
+ * in which every system runs the band-resident PCG on its own share of the
+ * SMs (the spare ones go to the system that would end last).  Otherwise, FP64: the batched streaming PCG -- every
  * system's iterations in the same two launches (each system its own blocks,
  * threads in proportion to its nodes, its own scalars; a system's blocks
  * return once it is done), chunks of 32 iterations replayed from a CUDA

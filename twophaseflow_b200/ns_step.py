@@ -14,7 +14,7 @@ holds the whole step, the solve included (its iteration count is read after
 the replay).  With the GMRES route it replays graph 1 (everything up to the
 PPE right-hand side), runs the host-driven solve, then replays graph 2
 (corrector, pressure update, CFL maxima).  The first call for a given dt runs
-the step eagerly (CCD plans, autotuning, allocator pools) and then captures.
+the step eagerly (CCD plans, launch-shape tuning, allocator pools) and then captures.
 With the quick-start selection the composition is pinned to six steps of the
 reference's own pipeline; ``save_checkpoint`` / ``restore_checkpoint_state``
 carry its state through the reference's restart format
