@@ -501,7 +501,9 @@ int tpf_ppe_solve(tpf_ppe* h, const double* rhs, const double* rho, double* p,
  * and all their ranges fit on chip at once (the systems' nodes summing to at
  * most ~400 000 in FP64, ~640 000 mixed, on 148 SMs): ONE cooperative launch
  * in which every system runs the band-resident PCG on its own share of the
- * SMs (the spare ones go to the system that would end last).  Otherwise, FP64: the batched streaming PCG -- every
+ * SMs (the spare ones go to the system that would end last).  Systems that
+ * fit one by one but not all at once (FP64) run as groups that do, one launch
+ * after the other.  Otherwise, FP64: the batched streaming PCG -- every
  * system's iterations in the same two launches (each system its own blocks,
  * threads in proportion to its nodes, its own scalars; a system's blocks
  * return once it is done), chunks of 32 iterations replayed from a CUDA

@@ -954,7 +954,8 @@ int launch_chunk(const tpf_ccd_plan* p, CcdArgs a, bool per, bool contig, const 
       return per ? ccd_chunk_contig_kernel<T, kChunkR, true, PL> : ccd_chunk_contig_kernel<T, kChunkR, false, PL>;
     };
     auto kern = plain ? pick(std::true_type{}) : pick(std::false_type{});
-    TPF_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    if (sh.smem > 48 * 1024)   // more than a launch may use unasked
+      TPF_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     kern<<<sh.blocks, sh.threads, sh.smem, s>>>(a, *K, g, Q, sh.pitch, vec ? 1 : 0);
   } else {
     auto pick = [&](auto epi, auto st) {
@@ -967,7 +968,7 @@ int launch_chunk(const tpf_ccd_plan* p, CcdArgs a, bool per, bool contig, const 
                 : a.vd_out ? pick2(std::integral_constant<int, kChunkVd>{})
                 : a.J      ? pick2(std::integral_constant<int, kChunkMetric>{})
                            : pick2(std::integral_constant<int, kChunkPlain>{});
-    if (sh.staged) TPF_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    if (sh.smem > 48 * 1024) TPF_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     kern<<<sh.blocks, sh.threads, sh.smem, s>>>(a, *K, g, Q);
   }
   TPF_CUDA_TRY(cudaGetLastError());
@@ -1223,9 +1224,8 @@ int tpf_ccd_plan_create(tpf_ccd_plan** out, int64_t n_pts, double h, int bc, int
   p->bc = bc;
   p->dtype = dtype;
   p->n_rows = (bc == TPF_BC_WALL) ? (int)(n_pts - 2) : (int)(n_pts - 1);
-  // chunk length = rows per lane of the warp kernel (8; 1, 2 or 4 warps per
-  // line up to 1024 rows); longer lines use the shared-memory chunk kernel
-  // with C = ceil(n_rows / 32)
+  // chunk length of ccd_line_kernel's tables: 8 rows up to 1024, else a 32nd of
+  // the line
   p->C = p->n_rows <= 1024 ? 8 : (p->n_rows + 31) / 32;
   std::vector<double> tab;
   int st = build_tables(p, tab);

@@ -3272,6 +3272,30 @@ bool band_batch_plan(tpf_ppe* const* hs, int n, bool mixed, std::vector<int>& nb
   return true;
 }
 
+// FP64 systems whose ranges fit on chip, but not all at once: groups that do,
+// largest systems first, so that a group's systems end at about the same time
+// (32 systems of 128^2..512^2: 101 ms in groups, 211 one after the other,
+// 260 as batched streaming PCG; 5 of 400^2..600^2: 49 against 54 one after the other).  Empty if some system does not fit by itself.
+std::vector<std::vector<int>> band_groups(tpf_ppe* const* hs, int n) {
+  std::vector<int> order(n);
+  std::iota(order.begin(), order.end(), 0);
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return hs[a]->g.ndof > hs[b]->g.ndof; });
+  std::vector<std::vector<int>> groups;
+  std::vector<tpf_ppe*> sub;
+  std::vector<int> nb(n), nmax(n);
+  size_t smem = 0;
+  for (int c : order) {
+    sub.push_back(hs[c]);
+    if (groups.empty() || !band_batch_plan(sub.data(), (int)sub.size(), false, nb, nmax, smem)) {
+      sub.assign(1, hs[c]);
+      if (!band_batch_plan(sub.data(), 1, false, nb, nmax, smem)) return {};
+      groups.emplace_back();
+    }
+    groups.back().push_back(c);
+  }
+  return groups;
+}
+
 // Batched streaming PCG (FP64 systems too large to keep resident): per system
 // the right-hand side, the initial residual and the first iteration as the
 // single-system launches, then chunks of kCgsChunk iterations of ALL systems
@@ -3480,8 +3504,8 @@ int tpf_ppe_solve_batched(tpf_ppe* const* hs, int n, const double* const* rhs, c
         if (int e = tpf_ppe_prepare(hs[c], rho[c], stream)) return e;
     return TPF_OK;
   };
-  // the band-resident batch where every band fits at once, else the
-  // all-global persistent body
+  // the band-resident batch where every range fits at once, in groups where each
+  // fits (FP64), else the batched streaming PCG (FP64) or the all-global body
   std::vector<int> bnb(n), bnmax(n);
   size_t bsmem = 0;
   bool force_band = false;
@@ -3494,12 +3518,33 @@ int tpf_ppe_solve_batched(tpf_ppe* const* hs, int n, const double* const* rhs, c
   std::vector<BandOutcome> out(n);
   const bool refused = force_stream && (force_band || force_global || mixed);
   const bool band = !force_stream && band_batch_plan(hs, n, mixed, bnb, bnmax, bsmem);
-  if (!band && (st = prepare())) return st;   // the band-resident batch prepares in its own setup
+  std::vector<std::vector<int>> groups;
+  if (!band && !mixed && !force_band && !force_global && !force_stream) groups = band_groups(hs, n);
+  if (!band && groups.empty() && (st = prepare())) return st;   // a band-resident batch prepares in its own setup
   TPF_CHECK_ARG(!(refused && !mixed), "conflicting CG kernel choices in one batch");
   TPF_CHECK_ARG(!refused, "the batched streaming PCG runs FP64 systems");
   if (force_stream) return solve_cgs_batch(hs, n, rhs, p, s, results);
   if (band) {
     if ((st = solve_band_batch(hs, n, rhs, rho, p, mixed, bnb, bnmax, bsmem, s, out.data()))) return st;
+  } else if (!groups.empty()) {
+    for (const auto& grp : groups) {
+      const int m = (int)grp.size();
+      std::vector<tpf_ppe*> gh(m);
+      std::vector<const double*> gr(m), gd(m);
+      std::vector<double*> gp(m);
+      std::vector<BandOutcome> go(m);
+      for (int k = 0; k < m; ++k) {
+        gh[k] = hs[grp[k]];
+        gr[k] = rhs[grp[k]];
+        gd[k] = rho ? rho[grp[k]] : nullptr;
+        gp[k] = p[grp[k]];
+      }
+      if (!band_batch_plan(gh.data(), m, false, bnb, bnmax, bsmem)) return TPF_EINVAL;   // it held in band_groups
+      if ((st = solve_band_batch(gh.data(), m, gr.data(), gd.data(), gp.data(), false, bnb, bnmax, bsmem, s,
+                                 go.data())))
+        return st;
+      for (int k = 0; k < m; ++k) out[grp[k]] = go[k];
+    }
   } else if (force_band) {
     tpf::set_error("the band-resident batch needs 2-D systems whose bands all fit in shared memory at once");
     return TPF_EINVAL;

@@ -531,10 +531,10 @@ def smoother_case(N, sweeps=256, block=4):
 
 def batched_case(n_cases=32, nmin=128, nmax=512, reps=3, seed=0, tol=1e-8):
     """``n_cases`` independent 2-D droplet PPEs with seeded uneven grids
-    (N_x, N_y uniform in [nmin, nmax]) solved in ONE persistent launch
-    (solve_batched) against one solve after the other (each on the whole
-    GPU, band-resident where it fits).  The batch is band-resident when the
-    bands of all cases fit in shared memory at once, else all-global."""
+    (N_x, N_y uniform in [nmin, nmax]) solved by solve_batched against one
+    solve after the other (each on the whole GPU, band-resident where it
+    fits).  The batch is band-resident, in one launch when all cases fit on
+    chip at once, else in groups that do."""
     import numpy as np
     import torch
     from . import PPESolverFVMMatrixFree, UniformGrid, solve_batched
