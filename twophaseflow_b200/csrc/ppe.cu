@@ -2157,6 +2157,7 @@ namespace {
 template <typename T>
 int dalloc(tpf_ppe* h, T** p, size_t n) {
   if (cudaMalloc(reinterpret_cast<void**>(p), std::max<size_t>(n, 1) * sizeof(T)) != cudaSuccess) {
+    cudaGetLastError();   // taken here, or the next call's launch check would find it
     tpf::set_error("cudaMalloc of %zu bytes failed", n * sizeof(T));
     return TPF_ECUDA;
   }
@@ -3455,10 +3456,6 @@ int solve_band_batch(tpf_ppe* const* hs, int n, const double* const* rhs, const 
     y.st = h->st;
     b->first[c + 1] = b->first[c] + nb[c];
     u->first[c + 1] = u->first[c] + std::min(h->ew_blocks, std::max(1, (h->g.ndof + 511) / 512));
-    if (y.prep.rho) {
-      h->line_ready = 0;
-      h->prepared = true;
-    }
   }
   tpf_ppe* h0 = hs[0];
   if (h0->batch_out_len < n) {
@@ -3477,6 +3474,11 @@ int solve_band_batch(tpf_ppe* const* hs, int n, const double* const* rhs, const 
   TPF_CUDA_TRY(cudaGetLastError());
   TPF_CUDA_TRY(cudaMemcpyAsync(out, h0->batch_out, sizeof(BandOutcome) * (size_t)n, cudaMemcpyDeviceToHost, s));
   TPF_CUDA_TRY(cudaStreamSynchronize(s));
+  for (int c = 0; c < n; ++c)
+    if (rho && rho[c]) {
+      hs[c]->line_ready = 0;
+      hs[c]->prepared = true;
+    }
   return TPF_OK;
 }
 
@@ -3524,6 +3526,9 @@ int tpf_ppe_solve_batched(tpf_ppe* const* hs, int n, const double* const* rhs, c
   TPF_CHECK_ARG(!(refused && !mixed), "conflicting CG kernel choices in one batch");
   TPF_CHECK_ARG(!refused, "the batched streaming PCG runs FP64 systems");
   if (force_stream) return solve_cgs_batch(hs, n, rhs, p, s, results);
+  if (band || !groups.empty())   // set again by solve_band_batch, once the new couplings are there
+    for (int c = 0; c < n; ++c)
+      if (rho && rho[c]) hs[c]->prepared = false;
   if (band) {
     if ((st = solve_band_batch(hs, n, rhs, rho, p, mixed, bnb, bnmax, bsmem, s, out.data()))) return st;
   } else if (!groups.empty()) {
