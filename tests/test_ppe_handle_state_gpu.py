@@ -77,3 +77,19 @@ def test_failed_batch_leaves_no_system_prepared_for_a_density_it_did_not_see(cud
         torch.cuda.synchronize()
         ref = _system(tuple(n - 1 for n in rho.shape), 3, cuda_device)[0].solve(x[2], rho)
         assert torch.equal(x[3], ref)
+
+
+def test_refused_batch_has_prepared_the_systems_before_the_refused_one(cuda_device):
+    """A system without couplings and without a density refuses the batch; the
+    systems before it were given their densities and solve for them."""
+    import torch
+    lib = _lib.load()
+    stream = torch.cuda.current_stream()
+    a, b = _system((30, 30), 3, cuda_device), _system((26, 41), 5, cuda_device)
+    first = torch.full_like(a[1], 1.0)
+    assert _solve(lib, a, first, stream) == _lib.TPF_OK
+    assert _batch(lib, [a, b], [a[1], None], stream) == _lib.TPF_EINVAL
+    assert _solve(lib, a, None, stream) == _lib.TPF_OK
+    torch.cuda.synchronize()
+    ref = _system((30, 30), 3, cuda_device)
+    assert torch.equal(a[3], ref[0].solve(ref[2], ref[1]))

@@ -3493,19 +3493,25 @@ int tpf_ppe_solve_batched(tpf_ppe* const* hs, int n, const double* const* rhs, c
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   int st;
   const bool mixed = hs[0]->o.precision == TPF_PREC_MIXED;
-  for (int c = 0; c < n; ++c) {
-    tpf_ppe* h = hs[c];
+  auto check = [&](int c) -> int {
+    const tpf_ppe* h = hs[c];
     TPF_CHECK_ARG(h && rhs[c] && p[c], "NULL handle or array for system %d", c);
     TPF_CHECK_ARG(h->o.method == TPF_PPE_CG, "batched solves run the CG route (system %d)", c);
     TPF_CHECK_ARG((h->o.precision == TPF_PREC_MIXED) == mixed, "all systems of a batch share one precision");
     TPF_CHECK_ARG(h->prepared || (rho && rho[c]), "operator coefficients of system %d are not initialised", c);
-  }
-  auto prepare = [&]() -> int {   // the couplings, one system after the other
-    for (int c = 0; c < n; ++c)
+    return TPF_OK;
+  };
+  auto prepare = [&](int systems) -> int {   // the couplings of the first ones, one system after the other
+    for (int c = 0; c < systems; ++c)
       if (rho && rho[c])
         if (int e = tpf_ppe_prepare(hs[c], rho[c], stream)) return e;
     return TPF_OK;
   };
+  for (int c = 0; c < n; ++c)
+    if ((st = check(c))) {   // the systems before the refused one have their densities
+      const int e = prepare(c);
+      return e ? e : st;
+    }
   // the band-resident batch where every range fits at once, in groups where each
   // fits (FP64), else the batched streaming PCG (FP64) or the all-global body
   std::vector<int> bnb(n), bnmax(n);
@@ -3522,7 +3528,7 @@ int tpf_ppe_solve_batched(tpf_ppe* const* hs, int n, const double* const* rhs, c
   const bool band = !force_stream && band_batch_plan(hs, n, mixed, bnb, bnmax, bsmem);
   std::vector<std::vector<int>> groups;
   if (!band && !mixed && !force_band && !force_global && !force_stream) groups = band_groups(hs, n);
-  if (!band && groups.empty() && (st = prepare())) return st;   // a band-resident batch prepares in its own setup
+  if (!band && groups.empty() && (st = prepare(n))) return st;   // a band-resident batch prepares in its own setup
   TPF_CHECK_ARG(!(refused && !mixed), "conflicting CG kernel choices in one batch");
   TPF_CHECK_ARG(!refused, "the batched streaming PCG runs FP64 systems");
   if (force_stream) return solve_cgs_batch(hs, n, rhs, p, s, results);
