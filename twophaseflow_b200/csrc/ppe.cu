@@ -3039,8 +3039,9 @@ int tpf_ppe_create(tpf_ppe** out, int ndim, const int64_t* N, const double* cons
   if ((st = dalloc(h, &h->st, 1))) return fail(st);
   if ((st = dalloc(h, &h->gst, 1))) return fail(st);
   {
-    // the streaming-PCG scalars and the private capture stream exist before
-    // any solve, so a first solve inside a stream capture allocates nothing
+    // the streaming-PCG scalars, the private capture stream and the exchange
+    // slots of the FP64 kernels exist before any solve, so a first solve inside a
+    // stream capture allocates nothing
     CgScal* c = nullptr;
     if ((st = dalloc(h, &c, 1))) return fail(st);
     h->cgs = c;
@@ -3051,6 +3052,8 @@ int tpf_ppe_create(tpf_ppe** out, int ndim, const int64_t* N, const double* cons
       return fail(TPF_ECUDA);
     }
     if ((st = dalloc(h, &h->march_slots, (size_t)2 * kMarchGrid * kBandLine))) return fail(st);
+    BandPlan bp;
+    if (band_plan(h, bp, false) && (st = ensure_band_buffers(h, bp.grid, false))) return fail(st);
   }
   *out = h;
   return TPF_OK;
