@@ -82,3 +82,21 @@ def test_zero_rhs_and_exhausted_cycles(cuda_device):
     s = _solver(N, pseudo_maxiter=1, ppe_restart=5)
     with pytest.raises(RuntimeError):
         s.solve(divergence_rhs(N, seed=4), rho)
+
+
+@pytest.mark.parametrize("N", [(24, 20), (700, 600)])
+def test_no_cycle_allowed_is_not_converged(cuda_device, N):
+    """With no restart cycle allowed the initial guess is not looked at: not
+    converged after no iterations and no operator application, even where the
+    guess is the solution (one launch, and the column kernels)."""
+    import torch
+    s = _solver(N, pseudo_tol=1e-3, pseudo_maxiter=0)
+    rho = torch.from_numpy(bubble_density(N, rho_g=0.1)).to(cuda_device)
+    x = torch.from_numpy(divergence_rhs(N, seed=3)).to(cuda_device)
+    x.view(-1)[s._pin_dof] = 0.0
+    s.prepare_operator(rho)
+    rhs = s.apply(x)
+    with pytest.raises(RuntimeError, match="info=0"):
+        s.solve(rhs, rho, 0.0, x)
+    assert s.last_diagnostics["ppe_low_order_gmres_iterations"] == 0
+    assert s.last_diagnostics["ppe_low_order_gmres_applies"] == 0

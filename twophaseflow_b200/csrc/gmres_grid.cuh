@@ -524,7 +524,9 @@ __global__ void __launch_bounds__(kGgThreads, 1) gmres_grid_kernel(const __grid_
   precondition([] {});
   const double mb = norm(square(z), nullptr);
   double factor = 1.0, ptol = mb * fmin(factor, atol / bnrm2);
-  if (ok && a.x_nonzero) {
+  if (a.maxiter == 0) {
+    // no cycle, and as in SciPy no look at the initial guess either
+  } else if (ok && a.x_nonzero) {
     rnorm = residual();
     ++applies;
     converged = rnorm < atol;
