@@ -100,3 +100,47 @@ def test_no_cycle_allowed_is_not_converged(cuda_device, N):
         s.solve(rhs, rho, 0.0, x)
     assert s.last_diagnostics["ppe_low_order_gmres_iterations"] == 0
     assert s.last_diagnostics["ppe_low_order_gmres_applies"] == 0
+
+
+# just below the sizes where a block's line factors no longer fit beside the Hessenberg matrix: 440^2 at restart 80,
+# 512^2 at 60; the longest lines without factors; the basis is in global memory throughout
+@pytest.mark.parametrize("N,kw", [((440, 440), dict(ppe_restart=80)), ((512, 512), dict(ppe_restart=30)),
+                                  ((512, 512), dict(ppe_restart=60)),
+                                  ((540, 540), dict(ppe_restart=80, ppe_preconditioner="jacobi")),
+                                  ((543, 530), dict(ppe_restart=30, ppe_preconditioner="none"))])
+def test_one_cycle_of_the_largest_systems(cuda_device, N, kw):
+    """One restart cycle against the oracle's: the iterate within 1e-8 of its
+    largest value (the least-squares problem of a cycle amplifies the round-off
+    of two orthogonalizations, some 1e-14, by at most the Hessenberg matrix'
+    condition, some 1e4 here), the residual within 1e-8."""
+    import torch
+    from twophaseflow_b200 import _lib
+    s = _solver(N, pseudo_tol=1e-12, pseudo_maxiter=1, **kw)
+    rho, rhs = bubble_density(N, rho_g=0.1), divergence_rhs(N, seed=4)
+    rho_d, rhs_d = torch.from_numpy(rho).to(cuda_device), torch.from_numpy(rhs).to(cuda_device)
+    p, res = torch.empty_like(rhs_d), _lib.tpf_ppe_result()
+    assert s.lib.tpf_ppe_solve(s._handle, _lib.dptr(rhs_d), _lib.dptr(rho_d), _lib.dptr(p), None,
+                               _lib.current_stream_handle(), res) == _lib.TPF_ENOCONV
+    assert res.iterations == s.restart
+    o = oppe.FVMMatrixFree(oppe.uniform_coords(N, (1.0, 1.0)), method="gmres", preconditioner=s.preconditioner)
+    o.prepare_operator(rho)
+    pco = oppe.line_precond_coeffs(o.coeffs, rho, o.c_tau, o.h_min)
+    dinv = oppe.jacobi_diag_inv(o.coeffs, o.pin)
+
+    def precondition(r):
+        r = r.reshape(o.shape)
+        if s.preconditioner == "line_pcr":
+            return oppe.line_precond(r, pco, o.pin, None).ravel()
+        z = r * dinv if s.preconditioner == "jacobi" else r.copy()
+        if s.preconditioner == "jacobi":
+            z.ravel()[o.pin] = 0.0
+        return z.ravel()
+    b = rhs.ravel().copy()
+    b[o.pin] = 0.0
+    x, _, its = oppe.gmres(lambda v: o.apply(v.reshape(o.shape)).ravel(), precondition, b, np.zeros_like(b), 1e-12,
+                           s.restart, 1)
+    assert its == s.restart
+    rel = np.linalg.norm(b - o.apply(x.reshape(o.shape)).ravel()) / np.linalg.norm(b)
+    x[o.pin] = 0.0
+    assert np.abs(p.cpu().numpy().ravel() - x).max() <= 1e-8 * np.abs(x).max()
+    assert abs(res.rel_residual - rel) <= 1e-8 * rel

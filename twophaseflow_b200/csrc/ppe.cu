@@ -2314,9 +2314,14 @@ struct GmresGridPlan {
 // Applies to 2-D systems whose lines fit a warp (544 nodes) and whose rows,
 // line factors and Hessenberg matrix fit the shared memory of one SM per
 // block; a block has up to a node per thread in whole rows, or what 148 blocks
-// need.  Up to that limit it is the faster side throughout (33^2: 14 us a column
-// against 57 as kernels, 129 x 97: 13 against 65, 201^2: 23 against 81); at
-// 513^2 the line factors of a block no longer fit and the kernels run (190 us).
+// need.  The limit depends on the restart length m, whose Hessenberg matrix
+// takes 4 m^2 bytes: with the line preconditioner 512^2 fits up to m = 67 and
+// 480^2 up to 84, without its factors 540^2 up to 166.  At that limit the basis
+// is in global memory and the kernel is still the faster side.  us a column,
+// kernels -> here: line preconditioner, m = 80: 64^2 58 -> 13, 200^2 84 -> 25,
+// 300^2 120 -> 41, 400^2 150 -> 57, 480^2 184 -> 113; 512^2 163 -> 97 at m = 60
+// and 125 -> 71 at m = 30; Jacobi, m = 80: 200^2 57 -> 20, 400^2 93 -> 47,
+// 512^2 131 -> 99, 540^2 139 -> 109, at m = 30 62 -> 51.
 bool gmres_grid_plan(const tpf_ppe* h, GmresGridPlan& P) {
   const Grid3& g = h->g;
   if (h->ndim != 2 || g.N2 != 0 || h->o.precond == TPF_PRECOND_LINE_PCR) return false;
