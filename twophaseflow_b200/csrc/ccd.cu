@@ -67,8 +67,9 @@ struct ChunkConst {
   T A[4], AR[4], B[4], BR[4];     // A (scaled) and B, and their R-th powers
   T P[4], Z[4];                   // P (scaled), P_last P^-1
   T Gf[4], Gb[4], AL[4], BL[4];   // periodic: ring closures, A and B to the power of the last chunk's rows
-  T cl[4], cr[4];                 // closure -> first right-hand side (scaled) / last solution
-  double Ml[4], Mr[4], cIl[4], cIr[4], cII[6];   // wall closures
+  // walls, in FP64 for FP32 too: the closures are evaluated in it
+  double cl[4], cr[4];            // closure -> first right-hand side (scaled) / last solution
+  double Ml[4], Mr[4], cIl[4], cIr[4], cII[6];
 };
 
 // Table layout (doubles).  C = chunk length, H0 = rows [0, H0) of the wall
@@ -606,7 +607,7 @@ ChunkConst<T, R> cast_chunk(const ChunkConst<double, R>& d) {
   auto cp = [](const double* a, T* b, int n) { for (int k = 0; k < n; ++k) b[k] = (T)a[k]; };
   cp(d.A, o.A, 4); cp(d.AR, o.AR, 4); cp(d.B, o.B, 4); cp(d.BR, o.BR, 4);
   cp(d.P, o.P, 4); cp(d.Z, o.Z, 4); cp(d.Gf, o.Gf, 4); cp(d.Gb, o.Gb, 4); cp(d.AL, o.AL, 4); cp(d.BL, o.BL, 4);
-  cp(d.cl, o.cl, 4); cp(d.cr, o.cr, 4);
+  std::copy(d.cl, d.cl + 4, o.cl); std::copy(d.cr, d.cr + 4, o.cr);
   std::copy(d.Ml, d.Ml + 4, o.Ml); std::copy(d.Mr, d.Mr + 4, o.Mr);
   std::copy(d.cIl, d.cIl + 4, o.cIl); std::copy(d.cIr, d.cIr + 4, o.cIr); std::copy(d.cII, d.cII + 6, o.cII);
   return o;

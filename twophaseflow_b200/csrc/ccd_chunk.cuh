@@ -89,8 +89,8 @@ __device__ __forceinline__ void chunk_solve(const ChunkConst<T, R>& K, const T (
     w[r] = {d1 + d0, d1 - d0};
     d0 = d1;
     if (!PERIODIC && r == 0 && q == 0) {
-      w[0].a -= (T)((double)K.cl[0] * bl0 + (double)K.cl[1] * bl1);
-      w[0].b -= (T)((double)K.cl[2] * bl0 + (double)K.cl[3] * bl1);
+      w[0].a -= (T)(K.cl[0] * bl0 + K.cl[1] * bl1);
+      w[0].b -= (T)(K.cl[2] * bl0 + K.cl[3] * bl1);
     }
     y = r == 0 ? w[0] : cmv(K.A, y, w[r]);
   }
@@ -131,8 +131,8 @@ __device__ __forceinline__ void chunk_solve(const ChunkConst<T, R>& K, const T (
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       if (!PERIODIC && r == cnt - 1) {
-        w[r] = cmv(K.Z, w[r], V2<T>{-(T)((double)K.cr[0] * br0 + (double)K.cr[1] * br1),
-                                    -(T)((double)K.cr[2] * br0 + (double)K.cr[3] * br1)});
+        w[r] = cmv(K.Z, w[r], V2<T>{-(T)(K.cr[0] * br0 + K.cr[1] * br1),
+                                    -(T)(K.cr[2] * br0 + K.cr[3] * br1)});
       }
       if (r >= cnt) w[r] = zero;
     }
