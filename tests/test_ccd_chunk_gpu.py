@@ -102,3 +102,61 @@ def test_one_bad_value_reaches_its_whole_line(cuda_device, bad, bc, axis):
         assert not bool(finite[:, 200].any())
         finite[:, 200] = True
         assert bool(finite.all())
+
+
+# many lines of lengths at which a block takes 24, 12, 6 and 3 lines (FP64) and, in FP32 with its blocks of up to 1024
+# threads, 28, 24, 32, 28, 24, 16, 12, 8, 6 and 4; longer lines than the chunk kernels take; rows that start off 16 bytes
+MANY = [((290, 135, 141), 0), ((135, 330, 141), 1), ((400, 135, 141), 0), ((560, 101, 165), 0), ((99, 660, 145), 1),
+        ((1000, 75, 127), 0), ((1340, 75, 97), 0), ((2000, 50, 97), 0), ((37, 2700, 97), 1), ((4097, 25, 97), 0),
+        ((4200, 7, 101), 0)]
+
+
+@pytest.mark.parametrize("shape,axis", MANY)
+@pytest.mark.parametrize("bc", ["wall", "periodic"])
+@pytest.mark.parametrize("dtype", ["f64", "f32"])
+def test_lines_per_block_do_not_enter_a_line(cuda_device, shape, axis, bc, dtype):
+    """Each line of a large field has the bits of its own solve among seven
+    lines, at the edges of a tile and in the last, ragged one."""
+    import torch
+    from twophaseflow_b200 import CCDSolver, UniformGrid
+    dt = torch.float64 if dtype == "f64" else torch.float32
+    f = torch.randn(shape, device=cuda_device, dtype=dt, generator=torch.Generator(device="cuda").manual_seed(4))
+    n = shape[axis]
+    if bc == "periodic":
+        f.select(axis, n - 1).copy_(f.select(axis, 0))
+    N = tuple(s - 1 for s in shape)
+    d = CCDSolver(UniformGrid(N), None, bc_type=bc, dtype=dt).differentiate(f, axis)
+    one = CCDSolver(UniformGrid((n - 1, 6), (1.0, 1.0)), None, bc_type=bc, dtype=dt)
+    lines = [t.movedim(axis, 0).reshape(n, -1) for t in (f, *d)]
+    m = lines[0].shape[1]
+    for c in (0, 9, 25, m // 2 - 3, m - 7):
+        cols = slice(c, c + 7)
+        e = one.differentiate(lines[0][:, cols].contiguous(), 0)
+        for k in range(2):
+            assert torch.equal(e[k], lines[1 + k][:, cols]), (c, k)
+
+
+def test_time_per_node_has_no_step_beyond_sixteen_chunks(cuda_device):
+    """Lines of 17 chunks fill 408 threads of an SM's 512 with 24 lines to a
+    block, lines of 16 all of them: at most 512 / 408 times as long a node (it
+    was 1.34 with 16 lines, 272 threads)."""
+    import torch
+    from twophaseflow_b200 import CCDSolver, UniformGrid
+    per_node = []
+    for n in (257, 273):
+        f = torch.randn((n, n, n), device=cuda_device, dtype=torch.float64)
+        ccd = CCDSolver(UniformGrid((n - 1,) * 3), None, bc_type="wall")
+        ccd.differentiate(f, 0)
+        times = []
+        for _ in range(7):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            torch.cuda.synchronize()
+            torch.cuda._sleep(200000)   # the calls are queued before the first one runs
+            a.record()
+            for _ in range(4):
+                ccd.differentiate(f, 0)
+            b.record()
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b))
+        per_node.append(min(times) / n**3)
+    assert per_node[1] <= 512 / 408 * per_node[0], per_node

@@ -115,6 +115,7 @@ struct CcdArgs {
   void* d2;
   int64_t outer, inner, n_lines;
   int n, n_rows, C, P, H0, TL, tl_shift;
+  int tl_inv;             // floor(2^16 / TL) + 1: x tl_inv >> 16 is x / TL for x <= 1024, TL <= 32
   int LS, FS;             // ybuf line stride / staged-f line stride (elements)
   int nbuf;               // f tile buffers (1 or 2)
   int n_tiles;
@@ -873,21 +874,48 @@ LaunchShape pick_shape(const tpf_ccd_plan* p, bool contig, int64_t n_lines) {
 
 // ---- chunk kernels: launch -------------------------------------------------------
 // How a call's lines are cut up: TL adjacent lines per block (0: a line is too
-// long for a block), `staged` for the strided axes, `pitch` of the contiguous
-// axis' lines in shared memory.  The results do not depend on any of them (each
-// line is solved by its own threads).
+// long for a block), `staged` and `wide` (up to 1024 threads) for the strided
+// axes, `pitch` of the contiguous axis' lines in shared memory.  The results do
+// not depend on any of them (each line is solved by its own threads).
 struct ChunkShape {
   int TL, threads, pitch;
-  bool staged;
+  bool staged, wide;
   size_t smem;
   unsigned blocks;
 };
 
-// The rule (one B200, FP64 unless said; us per call):
+// The rule (one B200, FP64 unless said; us per call).  What counts is how many
+// threads are resident on an SM, and then how long a run of adjacent lines a
+// block reads of each row:
 // * Strided axes: 16 lines, i.e. 128-byte rows; 32 where that keeps as many
 //   threads resident and the rows do not start on 32-byte sectors (257^3: 98.8
 //   against 108.9 on axis 0; 256^3 nodes, whose rows do: 89.0 against 81.7;
-//   129 x 97 x 162 axis 1, 480 resident threads against 384: 13.1 against 16.3).
+//   129 x 97 x 162 axis 1, 480 resident threads against 384: 13.1 against 16.3);
+//   not for FP64 lines of 11 to 14 chunks, where two blocks of 16 lines hold as
+//   many threads as one of 32 (209^3 53.4 against 60.2, 225^3 65.5 against 68.2,
+//   193^3 45 and 47; 241^3, 15 chunks, the other way, 93.5 against 81, and so the
+//   epilogues on walls, whose 128 registers spill, 193^3 108 against 103).
+//   Longer lines (more than 32 chunks) take fewer: half as many each time.
+// * Where such a block has more than half of the threads an SM holds in FP64, a
+//   second one does not fit beside it and half as many lines again keep more
+//   threads resident: 24, 12, 6 or 3, where there are several tiles per SM (axis
+//   0, wall: 273^3 134 against 160 with 16 lines, 300^3 153 against 182, 520 x
+//   200 x 200 149 against 180, 600 x 160 x 160 104 against 125; 2051^2 57 against
+//   62).  At 20 chunks and more of 16 lines, where rows do not start on a sector,
+//   20 are the better number on walls (321^3 221 with 20, 228 with 24, 242 with
+//   16; 385^3 the other way, 406 against 372) and 16 on periodic lines (321^3 198
+//   with 16, 209 with 20, 218 with 24; 320^3, aligned, 198 with 16, 178 with 24).
+// * FP32, d1 and d2 plainly stored: up to 1024 threads of 64 registers (a few
+//   spills on walls) instead of 512 of 74, where rows do not start on 16 bytes, so
+//   that short runs of them waste sectors, or a line has more than 64 chunks, of
+//   which 512 threads hold but 16 to 28 bytes of a row; again with several tiles
+//   per SM.  32 to 24 lines where two blocks fit, else the most that one holds
+//   (axis 0: 257^3 67 against 79, 273^3 93 against 108, 417^3 305 against 403,
+//   513^3 578 against 653, 1100 x 140 x 140 127 against 192, 2049 x 140 x 140 243
+//   against 387).  Elsewhere the spills cost more than the threads bring (340^3,
+//   aligned: 161 against 140; 193^3 in L2: 26 against 24), and so does the longer
+//   run on periodic lines whose rows lie close together (513^3 axis 1: 510
+//   against 469; axis 0, rows 1 MB apart: 536 against 570).
 // * Contiguous axis: 8 or 16 lines, whichever keeps more threads resident (193
 //   nodes: 45.3 with 8, 54.5 with 16; 162 nodes: 18.6 and 15.3).
 // * Fewer lines per block while that leaves half of the SMs without one, down
@@ -897,7 +925,7 @@ struct ChunkShape {
 //   193^3 45.3 against 57.9; 129 x 97 x 162 the other way, 14.1 against 13.1;
 //   FP32 191 x 160 x 225 29.5 against 19.6.
 template <typename T>
-ChunkShape chunk_shape(const tpf_ccd_plan* p, bool contig, int64_t n_lines, int64_t inner) {
+ChunkShape chunk_shape(const tpf_ccd_plan* p, bool contig, bool plain, int64_t n_lines, int64_t inner) {
   constexpr bool F64 = std::is_same<T, double>::value;
   const int Q = (p->n_rows + kChunkR - 1) / kChunkR, n = (int)p->n_pts, nsm = tpf::sm_count();
   ChunkShape s{};
@@ -914,19 +942,43 @@ ChunkShape chunk_shape(const tpf_ccd_plan* p, bool contig, int64_t n_lines, int6
   auto per_sm = [&](int tl) { return std::max(1, 65536 / ((F64 ? 128 : 96) * threads(tl))); };
   auto resident = [&](int tl) { return fits(tl) ? per_sm(tl) * tl * Q : 0; };
   auto tiles = [&](int tl) { return (n_lines + tl - 1) / tl; };
+  auto many = [&](int tl) { return tiles(tl) >= 4 * (int64_t)nsm; };
+  auto done = [&](int tl) {
+    s.TL = tl;
+    s.threads = threads(tl);
+    s.smem = smem(tl, s.staged);
+    s.blocks = (unsigned)(s.staged ? (int64_t)nsm * per_sm(tl) : tiles(tl));
+    return s;
+  };
+  const bool wall = p->bc == TPF_BC_WALL, ragged = (inner * sizeof(T)) % 16 != 0;
+  if (!F64 && !contig && plain &&
+      (Q > 64 || (ragged && (wall ? Q >= 14 : Q > 16 && inner * sizeof(T) >= 128 * 1024)))) {
+    int tl = 0;
+    for (int k : {24, 28, 32})   // two blocks of an SM's 1024 threads
+      if (k * Q <= 512) tl = k;
+    if (!tl)
+      for (int k : {4, 6, 8, 12, 16, 24, 28, 32})
+        if (k * Q <= 1024) tl = k;
+    if (tl && many(tl)) {
+      s.wide = true;
+      return done(tl);
+    }
+  }
   int TL = 16;
   if (contig) TL = resident(16) > resident(8) ? 16 : 8;
-  else if (resident(32) >= resident(16) && (inner * sizeof(T)) % 32 != 0 && tiles(32) >= nsm) TL = 32;
+  else if (resident(32) >= resident(16) && (inner * sizeof(T)) % 32 != 0 && tiles(32) >= nsm &&
+           !(F64 && Q > 10 && Q < 15 && (plain || !wall)))
+    TL = 32;
   while (TL > 2 && !fits(TL)) TL >>= 1;
   if (!fits(TL)) return s;
+  if (F64 && !contig && TL <= 16 && TL * Q > 256) {
+    int more = TL + TL / 2;
+    if (TL == 16 && Q > 19 && (inner * sizeof(T)) % 32 != 0) more = wall && Q < 23 ? 20 : TL;
+    if (more * Q <= 512 && many(more)) TL = more;
+  }
   while (TL > 2 && 2 * tiles(TL) <= nsm && TL / 2 * Q >= 128) TL >>= 1;
-  s.TL = TL;
-  s.threads = threads(TL);
-  const int64_t slots = (int64_t)nsm * per_sm(TL);
-  s.staged = !contig && F64 && tiles(TL) > 2 * slots && smem(TL, true) <= limit;
-  s.smem = smem(TL, s.staged);
-  s.blocks = (unsigned)(s.staged ? slots : tiles(TL));
-  return s;
+  s.staged = !contig && F64 && tiles(TL) > 2 * (int64_t)nsm * per_sm(TL) && smem(TL, true) <= limit;
+  return done(TL);
 }
 
 template <typename T>
@@ -935,6 +987,7 @@ int launch_chunk(const tpf_ccd_plan* p, CcdArgs a, bool per, bool contig, const 
   a.TL = sh.TL;
   a.tl_shift = 0;
   while ((1 << a.tl_shift) < sh.TL) ++a.tl_shift;
+  a.tl_inv = 65536 / sh.TL + 1;
   a.n_tiles = (int)((a.n_lines + sh.TL - 1) / sh.TL);
   const T* g;
   const ChunkConst<T, kChunkR>* K;
@@ -959,12 +1012,26 @@ int launch_chunk(const tpf_ccd_plan* p, CcdArgs a, bool per, bool contig, const 
       TPF_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     kern<<<sh.blocks, sh.threads, sh.smem, s>>>(a, *K, g, Q, sh.pitch, vec ? 1 : 0);
   } else {
-    auto pick = [&](auto epi, auto st) {
-      constexpr int E = decltype(epi)::value;
-      constexpr bool S = decltype(st)::value;
-      return per ? ccd_chunk_strided_kernel<T, kChunkR, true, E, S> : ccd_chunk_strided_kernel<T, kChunkR, false, E, S>;
+    auto pick = [&](auto epi, auto st, auto pow2, auto threads) {
+      constexpr int E = decltype(epi)::value, TH = decltype(threads)::value;
+      constexpr bool S = decltype(st)::value, P2 = decltype(pow2)::value;
+      return per ? ccd_chunk_strided_kernel<T, kChunkR, true, E, S, P2, TH>
+                 : ccd_chunk_strided_kernel<T, kChunkR, false, E, S, P2, TH>;
     };
-    auto pick2 = [&](auto epi) { return sh.staged ? pick(epi, std::true_type{}) : pick(epi, std::false_type{}); };
+    const bool pow2 = (sh.TL & (sh.TL - 1)) == 0;
+    using Yes = std::true_type;
+    using No = std::false_type;
+    using Few = std::integral_constant<int, 512>;
+    auto pick2 = [&](auto epi) {
+      constexpr int E = decltype(epi)::value;
+      if constexpr (std::is_same<T, double>::value) {
+        if (!pow2) return sh.staged ? pick(epi, Yes{}, No{}, Few{}) : pick(epi, No{}, No{}, Few{});
+        if (sh.staged) return pick(epi, Yes{}, Yes{}, Few{});
+      } else if constexpr (E == kChunkPlain) {
+        if (sh.wide) return pick(epi, No{}, No{}, std::integral_constant<int, 1024>{});
+      }
+      return pick(epi, No{}, Yes{}, Few{});
+    };
     auto kern = a.cr_out   ? pick2(std::integral_constant<int, kChunkCorrector>{})
                 : a.vd_out ? pick2(std::integral_constant<int, kChunkVd>{})
                 : a.J      ? pick2(std::integral_constant<int, kChunkMetric>{})
@@ -1013,7 +1080,7 @@ int launch_ccd(const tpf_ccd_plan* p, int64_t outer, int64_t inner, const void* 
   }
   const bool per = (p->bc == TPF_BC_PERIODIC) && !a.ovl && !a.ovr;
   if (per == (p->bc == TPF_BC_PERIODIC)) {
-    const ChunkShape sh = chunk_shape<T>(p, contig, n_lines, inner);
+    const ChunkShape sh = chunk_shape<T>(p, contig, !a.J && !a.vd_out && !a.cr_out, n_lines, inner);
     if (sh.TL > 0) return launch_chunk<T>(p, a, per, contig, sh, stream);
   }
   // longer lines, and closure overrides on a periodic plan

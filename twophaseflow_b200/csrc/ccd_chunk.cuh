@@ -359,13 +359,16 @@ __device__ __forceinline__ void chunk_load(const CcdArgs& a, const ChunkConst<T,
 // L0 + l (lanes on adjacent lines).  STAGED: a block takes several tiles of TL
 // lines in turn and copies the next tile's f into shared memory while it
 // solves the present one; otherwise a block has one tile and a thread loads its
-// rows straight into registers.
-template <typename T, int R, bool PERIODIC, int EPI, bool STAGED>
-__global__ void __launch_bounds__(512)
+// rows straight into registers.  POW2: TL is a power of two (the division by any
+// other TL costs a block's start 2 %, FP32 epilogues 6-9 %).  THREADS: most
+// threads of a block, 512 or (FP32, 64 registers a thread) 1024.
+template <typename T, int R, bool PERIODIC, int EPI, bool STAGED, bool POW2, int THREADS>
+__global__ void __launch_bounds__(THREADS)
     ccd_chunk_strided_kernel(const __grid_constant__ CcdArgs a, const __grid_constant__ ChunkConst<T, R> K,
                              const T* __restrict__ gtab, int Q) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int t = threadIdx.x, TL = a.TL, q = t >> a.tl_shift, l = t & (TL - 1);
+  const int t = threadIdx.x, TL = a.TL;
+  const int q = POW2 ? t >> a.tl_shift : t * a.tl_inv >> 16, l = POW2 ? t & (TL - 1) : t - q * TL;
   T* G = reinterpret_cast<T*>(smem_raw);
   T* e = G + 4 * (kChunkHead + R);
   T* poison = e + 4 * blockDim.x;   // [TL]
@@ -383,10 +386,10 @@ __global__ void __launch_bounds__(512)
     const unsigned o = (unsigned)L / (unsigned)inner;
     return (int64_t)o * n * inner + (L - (int64_t)o * inner);
   };
-  // rows q, q + rows, ... of the thread's line (all threads of the block take part)
-  const int rows = blockDim.x >> a.tl_shift;
+  // rows q, q + rows, ... of the thread's line (idle threads of the block take part)
+  const int rows = POW2 ? (int)blockDim.x >> a.tl_shift : (int)blockDim.x * a.tl_inv >> 16;
   auto fetch = [&](int64_t b) {
-    if (b >= 0) {
+    if (b >= 0 && (POW2 || q < rows)) {
       const T* src = static_cast<const T*>(a.f) + b + (int64_t)q * inner;
       const int64_t step = (int64_t)rows * inner;
       for (int k = q; k < n; k += rows, src += step) cp_async<sizeof(T)>(fs + k * TL + l, src, true);
