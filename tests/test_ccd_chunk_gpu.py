@@ -160,3 +160,118 @@ def test_time_per_node_has_no_step_beyond_sixteen_chunks(cuda_device):
             times.append(a.elapsed_time(b))
         per_node.append(min(times) / n**3)
     assert per_node[1] <= 512 / 408 * per_node[0], per_node
+
+
+class _Calls:
+    """The epilogues of the line solve along one axis, through the C ABI."""
+
+    def __init__(self, shape, axis, bc, dt, device):
+        import ctypes as C
+
+        import torch
+        from twophaseflow_b200 import _lib
+        from twophaseflow_b200.arrays import line_split
+        self.lib, self._lib = _lib.load(), _lib
+        g = torch.Generator(device="cuda").manual_seed(5)
+        self.f, self.u, drho = (torch.randn(shape, device=device, dtype=dt, generator=g) for _ in range(3))
+        self.rho, self.drho = torch.rand(shape, device=device, dtype=dt, generator=g) + 1, drho
+        n = shape[axis]
+        self.plan = C.c_void_p()
+        _lib.check(self.lib.tpf_ccd_plan_create(C.byref(self.plan), n, 1.0 / (n - 1),
+                                                _lib.TPF_BC_PERIODIC if bc == "periodic" else _lib.TPF_BC_WALL,
+                                                _lib.TPF_F64 if dt == torch.float64 else _lib.TPF_F32))
+        x = np.arange(n, dtype=np.float64)
+        J, dJ = 1.0 + 0.25 * np.sin(x), 0.5 * np.cos(x)
+        _lib.check(self.lib.tpf_ccd_plan_set_metric(self.plan, *(a.ctypes.data_as(C.POINTER(C.c_double)) for a in (J, dJ))))
+        outer, _, inner = line_split(shape, axis)
+        self.split = (outer, inner)
+
+    def __del__(self):
+        self.lib.tpf_ccd_plan_destroy(self.plan)
+
+    def run(self, kind, metric, out):
+        """out: the fields written (d1, d2), or the one written, which is the
+        corrector's u* too and what the variable-density term adds to."""
+        p, s = self._lib.dptr, self._lib.current_stream_handle()
+        flags = self._lib.TPF_CCD_APPLY_METRIC if metric else 0
+        if kind == "plain":
+            st = self.lib.tpf_ccd_apply(self.plan, *self.split, p(self.f), p(out[0]), p(out[1]), None, None, flags, s)
+        elif kind == "corrector":
+            st = self.lib.tpf_ccd_apply_corrector(self.plan, *self.split, p(self.f), p(out[0]), p(self.rho), 0.01,
+                                                  p(out[0]), flags, s)
+        else:
+            st = self.lib.tpf_ccd_apply_vd(self.plan, *self.split, p(self.f), p(self.rho), p(self.drho), p(out[0]), 1,
+                                           flags, s)
+        self._lib.check(st)
+
+
+# one warp's elements and less than a batch of them; several batches and a remainder; a ragged last tile; long lines
+@pytest.mark.parametrize("shape,axis", [((3, 7), 1), ((5, 33), 1), ((65, 65), 1), ((65, 65), 0), ((41, 130), 1),
+                                        ((37, 1500), 1), ((12, 11, 194), 2), ((30, 20, 9), 0), ((9, 50, 21), 1)])
+@pytest.mark.parametrize("bc", ["wall", "periodic"])
+@pytest.mark.parametrize("dtype", ["f64", "f32"])
+@pytest.mark.parametrize("metric", [False, True])
+def test_epilogues_against_the_plain_derivatives(cuda_device, shape, axis, bc, dtype, metric):
+    """Corrector (in place) and variable-density term (accumulated) equal the
+    formulas on the plain call's d1 and d2 to the rounding of the type, some
+    operations of 4 eps each; the metric is that of the chain rule."""
+    import torch
+    dt = torch.float64 if dtype == "f64" else torch.float32
+    c = _Calls(shape, axis, bc, dt, cuda_device)
+    if bc == "periodic":
+        c.f.select(axis, shape[axis] - 1).copy_(c.f.select(axis, 0))
+    d = [torch.empty_like(c.f) for _ in range(2)]
+    c.run("plain", False, d)
+    d1, d2 = (t.double() for t in d)
+    if metric:
+        x = torch.arange(shape[axis], device=cuda_device, dtype=torch.float64)
+        J, dJ = ((1.0 + 0.25 * torch.sin(x)), 0.5 * torch.cos(x))
+        J, dJ = (t.view([-1] + [1] * (len(shape) - 1 - axis)) for t in (J, dJ))
+        d2 = J * J * d2 + J * dJ * d1
+        d1 = J * d1
+        m = [torch.empty_like(c.f) for _ in range(2)]
+        c.run("plain", True, m)
+        for got, want in zip(m, (d1, d2)):
+            assert float((got.double() - want).abs().max()) <= 32 * torch.finfo(dt).eps * float(want.abs().max() + d1.abs().max())
+    rho, drho, u = c.rho.double(), c.drho.double(), c.u.double()
+    eps = 32 * torch.finfo(dt).eps
+    step = 0.01 / rho * d1
+    if bc == "wall":
+        step.select(axis, 0).zero_()
+        step.select(axis, shape[axis] - 1).zero_()
+    got = c.u.clone()
+    c.run("corrector", metric, [got])
+    assert float((got.double() - (u - step)).abs().max()) <= eps * float(u.abs().max() + step.abs().max())
+    term = d2 / rho - drho / (rho * rho) * d1
+    got = c.u.clone()
+    c.run("vd", metric, [got])
+    size = (d2 / rho).abs().max() + (drho / (rho * rho) * d1).abs().max()
+    assert float((got.double() - (u + term)).abs().max()) <= eps * float(u.abs().max() + size)
+
+
+@pytest.mark.parametrize("dtype", ["f64", "f32"])
+def test_epilogues_of_the_contiguous_axis_cost_their_bytes(cuda_device, dtype):
+    """The accumulated variable-density term moves 5 values a node where the
+    plain call moves 3: at most half as long again as that ratio says (it was
+    4.1 instead of 1.7 times as long when each element's operands were waited
+    for by themselves)."""
+    import torch
+    dt = torch.float64 if dtype == "f64" else torch.float32
+    c = _Calls((193, 193, 193), 2, "wall", dt, cuda_device)
+    out = [torch.zeros_like(c.f) for _ in range(2)]
+    times = {}
+    for kind in ("plain", "vd"):
+        c.run(kind, False, out)
+        best = []
+        for _ in range(7):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            torch.cuda.synchronize()
+            torch.cuda._sleep(200000)
+            a.record()
+            for _ in range(8):
+                c.run(kind, False, out)
+            b.record()
+            torch.cuda.synchronize()
+            best.append(a.elapsed_time(b))
+        times[kind] = min(best)
+    assert times["vd"] <= 1.5 * 5 / 3 * times["plain"], times
