@@ -136,30 +136,42 @@ def test_lines_per_block_do_not_enter_a_line(cuda_device, shape, axis, bc, dtype
             assert torch.equal(e[k], lines[1 + k][:, cols]), (c, k)
 
 
+def _ns_per_node(n, bc, device):
+    """FP64 differentiation of n^3 nodes along axis 0, the shortest of seven runs of four."""
+    import torch
+    from twophaseflow_b200 import CCDSolver, UniformGrid
+    f = torch.randn((n, n, n), device=device, dtype=torch.float64)
+    ccd = CCDSolver(UniformGrid((n - 1,) * 3), None, bc_type=bc)
+    ccd.differentiate(f, 0)
+    times = []
+    for _ in range(7):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        torch.cuda.synchronize()
+        torch.cuda._sleep(200000)   # the calls are queued before the first one runs
+        a.record()
+        for _ in range(4):
+            ccd.differentiate(f, 0)
+        b.record()
+        torch.cuda.synchronize()
+        times.append(a.elapsed_time(b))
+    return min(times) / 4 * 1e6 / n**3
+
+
 def test_time_per_node_has_no_step_beyond_sixteen_chunks(cuda_device):
     """Lines of 17 chunks fill 408 threads of an SM's 512 with 24 lines to a
     block, lines of 16 all of them: at most 512 / 408 times as long a node (it
     was 1.34 with 16 lines, 272 threads)."""
-    import torch
-    from twophaseflow_b200 import CCDSolver, UniformGrid
-    per_node = []
-    for n in (257, 273):
-        f = torch.randn((n, n, n), device=cuda_device, dtype=torch.float64)
-        ccd = CCDSolver(UniformGrid((n - 1,) * 3), None, bc_type="wall")
-        ccd.differentiate(f, 0)
-        times = []
-        for _ in range(7):
-            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-            torch.cuda.synchronize()
-            torch.cuda._sleep(200000)   # the calls are queued before the first one runs
-            a.record()
-            for _ in range(4):
-                ccd.differentiate(f, 0)
-            b.record()
-            torch.cuda.synchronize()
-            times.append(a.elapsed_time(b))
-        per_node.append(min(times) / n**3)
-    assert per_node[1] <= 512 / 408 * per_node[0], per_node
+    a, b = (_ns_per_node(n, "wall", cuda_device) for n in (257, 273))
+    assert b <= 512 / 408 * a, (a, b)
+
+
+def test_time_per_node_has_no_step_beyond_two_gigabytes(cuda_device):
+    """Field and derivatives of 449^3 nodes are 2.2 GB, of 417^3 1.7; both have
+    16 lines to a block, 448 and 416 threads, so the larger field should take no
+    longer a node: a tenth is left for the runs' scatter (it was 1.25 to 1.3
+    while the SMs took their tiles at a fixed stride and drifted apart)."""
+    a, b = (_ns_per_node(n, "periodic", cuda_device) for n in (417, 449))
+    assert b <= 1.1 * a, (a, b)
 
 
 class _Calls:

@@ -874,17 +874,18 @@ LaunchShape pick_shape(const tpf_ccd_plan* p, bool contig, int64_t n_lines) {
 
 // ---- chunk kernels: launch -------------------------------------------------------
 // How a call's lines are cut up: TL adjacent lines per block (0: a line is too
-// long for a block), `staged` and `wide` (up to 1024 threads) for the strided
-// axes, `pitch` of the contiguous axis' lines in shared memory.  The results do
+// long for a block), `staged`, `steal` and `wide` (up to 1024 threads) for the
+// strided axes, `pitch` of the contiguous axis' lines in shared memory.  The results do
 // not depend on any of them (each line is solved by its own threads).
 struct ChunkShape {
   int TL, threads, pitch;
-  bool staged, wide;
+  bool staged, steal, wide;
   size_t smem;
   unsigned blocks;
 };
 
-// The rule (one B200, FP64 unless said; us per call).  What counts is how many
+// The rule (one B200, FP64 unless said; us per call; plain: d1 and d2 stored as
+// they are, heavy: the corrector and variable-density epilogues).  What counts is how many
 // threads are resident on an SM, and then how long a run of adjacent lines a
 // block reads of each row:
 // * Strided axes: 16 lines, i.e. 128-byte rows; 32 where that keeps as many
@@ -924,8 +925,15 @@ struct ChunkShape {
 //   every resident block has more than two tiles: 257^3 98.8 against 112.5,
 //   193^3 45.3 against 57.9; 129 x 97 x 162 the other way, 14.1 against 13.1;
 //   FP32 191 x 160 x 225 29.5 against 19.6.
+// * Its tiles dealt out instead of taken by a fixed stride for fields of more than
+//   2 GB in and out and for up to 8 lines a block, from 22 chunks on (periodic
+//   449^3 491 against 678, 577^3 axis 0 1338 against 1760; wall 449^3 550 against
+//   577, 1025 x 140 x 140 154 against 170; 300^3 154 and 156; 600 x 161 x 161 the
+//   other way, 128 against 122).  Not walls of 29 to 32 chunks (481^3 805 against
+//   769), nor the heavy epilogues on walls, which it makes spill more (193^3 115
+//   against 105).
 template <typename T>
-ChunkShape chunk_shape(const tpf_ccd_plan* p, bool contig, bool plain, int64_t n_lines, int64_t inner) {
+ChunkShape chunk_shape(const tpf_ccd_plan* p, bool contig, bool plain, bool heavy, int64_t n_lines, int64_t inner) {
   constexpr bool F64 = std::is_same<T, double>::value;
   const int Q = (p->n_rows + kChunkR - 1) / kChunkR, n = (int)p->n_pts, nsm = tpf::sm_count();
   ChunkShape s{};
@@ -947,7 +955,7 @@ ChunkShape chunk_shape(const tpf_ccd_plan* p, bool contig, bool plain, int64_t n
     s.TL = tl;
     s.threads = threads(tl);
     s.smem = smem(tl, s.staged);
-    s.blocks = (unsigned)(s.staged ? (int64_t)nsm * per_sm(tl) : tiles(tl));
+    s.blocks = (unsigned)(s.staged && !s.steal ? (int64_t)nsm * per_sm(tl) : tiles(tl));
     return s;
   };
   const bool wall = p->bc == TPF_BC_WALL, ragged = (inner * sizeof(T)) % 16 != 0;
@@ -978,6 +986,8 @@ ChunkShape chunk_shape(const tpf_ccd_plan* p, bool contig, bool plain, int64_t n
   }
   while (TL > 2 && 2 * tiles(TL) <= nsm && TL / 2 * Q >= 128) TL >>= 1;
   s.staged = !contig && F64 && tiles(TL) > 2 * (int64_t)nsm * per_sm(TL) && smem(TL, true) <= limit;
+  const bool far = 3 * sizeof(T) * (double)n_lines * n > 2e9;   // in and out
+  s.steal = s.staged && Q > 21 && (far || TL <= 8) && !(wall && (heavy || (Q > 28 && Q < 33)));
   return done(TL);
 }
 
@@ -1012,25 +1022,29 @@ int launch_chunk(const tpf_ccd_plan* p, CcdArgs a, bool per, bool contig, const 
       TPF_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     kern<<<sh.blocks, sh.threads, sh.smem, s>>>(a, *K, g, Q, sh.pitch, vec ? 1 : 0);
   } else {
-    auto pick = [&](auto epi, auto st, auto pow2, auto threads) {
-      constexpr int E = decltype(epi)::value, TH = decltype(threads)::value;
-      constexpr bool S = decltype(st)::value, P2 = decltype(pow2)::value;
+    auto pick = [&](auto epi, auto stage, auto pow2, auto threads) {
+      constexpr int E = decltype(epi)::value, S = decltype(stage)::value, TH = decltype(threads)::value;
+      constexpr bool P2 = decltype(pow2)::value;
       return per ? ccd_chunk_strided_kernel<T, kChunkR, true, E, S, P2, TH>
                  : ccd_chunk_strided_kernel<T, kChunkR, false, E, S, P2, TH>;
     };
     const bool pow2 = (sh.TL & (sh.TL - 1)) == 0;
-    using Yes = std::true_type;
-    using No = std::false_type;
+    using Direct = std::integral_constant<int, kChunkDirect>;
     using Few = std::integral_constant<int, 512>;
     auto pick2 = [&](auto epi) {
       constexpr int E = decltype(epi)::value;
       if constexpr (std::is_same<T, double>::value) {
-        if (!pow2) return sh.staged ? pick(epi, Yes{}, No{}, Few{}) : pick(epi, No{}, No{}, Few{});
-        if (sh.staged) return pick(epi, Yes{}, Yes{}, Few{});
-      } else if constexpr (E == kChunkPlain) {
-        if (sh.wide) return pick(epi, No{}, No{}, std::integral_constant<int, 1024>{});
+        auto lines = [&](auto stage) {
+          return pow2 ? pick(epi, stage, std::true_type{}, Few{}) : pick(epi, stage, std::false_type{}, Few{});
+        };
+        if (sh.steal) return lines(std::integral_constant<int, kChunkSteal>{});
+        if (sh.staged) return lines(std::integral_constant<int, kChunkStride>{});
+        return lines(Direct{});
+      } else {
+        if constexpr (E == kChunkPlain)
+          if (sh.wide) return pick(epi, Direct{}, std::false_type{}, std::integral_constant<int, 1024>{});
+        return pick(epi, Direct{}, std::true_type{}, Few{});
       }
-      return pick(epi, No{}, Yes{}, Few{});
     };
     auto kern = a.cr_out   ? pick2(std::integral_constant<int, kChunkCorrector>{})
                 : a.vd_out ? pick2(std::integral_constant<int, kChunkVd>{})
@@ -1080,7 +1094,8 @@ int launch_ccd(const tpf_ccd_plan* p, int64_t outer, int64_t inner, const void* 
   }
   const bool per = (p->bc == TPF_BC_PERIODIC) && !a.ovl && !a.ovr;
   if (per == (p->bc == TPF_BC_PERIODIC)) {
-    const ChunkShape sh = chunk_shape<T>(p, contig, !a.J && !a.vd_out && !a.cr_out, n_lines, inner);
+    const bool heavy = a.vd_out || a.cr_out;
+    const ChunkShape sh = chunk_shape<T>(p, contig, !a.J && !heavy, heavy, n_lines, inner);
     if (sh.TL > 0) return launch_chunk<T>(p, a, per, contig, sh, stream);
   }
   // longer lines, and closure overrides on a periodic plan

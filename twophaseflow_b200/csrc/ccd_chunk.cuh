@@ -215,7 +215,13 @@ __device__ __forceinline__ void chunk_store(const CcdArgs& a, const ChunkConst<T
       o2 = Jk * Jk * o2 + Jk * dJk * o1;
       o1 = Jk * o1;
     }
-    store_out<T>(a, base + (int64_t)k * inner, o1, o2, k);
+    const int64_t gi = base + (int64_t)k * inner;
+    if constexpr (EPI == kChunkPlain || EPI == kChunkMetric) {   // without the others' registers
+      if (a.d1) static_cast<T*>(a.d1)[gi] = (T)o1;
+      if (a.d2) static_cast<T*>(a.d2)[gi] = (T)o2;
+    } else {
+      store_out<T>(a, gi, o1, o2, k);
+    }
   };
   const int64_t o0 = base + (int64_t)k0 * inner;
   if constexpr (EPI == kChunkPlain) {
@@ -374,18 +380,61 @@ __device__ __forceinline__ void chunk_load(const CcdArgs& a, const ChunkConst<T,
   }
 }
 
+enum { kChunkDirect = 0, kChunkStride = 1, kChunkSteal = 2 };
+
+// Tiles dealt out as blocks become free (kChunkSteal): the launch has a block per
+// tile, and a running block asks for the first one that has not started to be
+// cancelled and solves its tile instead (cluster launch control).  Like
+// a fixed stride through the tiles this lets a block copy its next tile early,
+// but the tiles in work stay next to each other.  With the stride the SMs drift
+// apart, and neighbouring tiles, which share the sectors at the ends of their
+// rows and the pages the rows lie in, no longer meet in the caches: fields of more
+// than 2 GB in and out took a third longer a node on axis 0 (periodic 417^3
+// 5.7 ns, 449^3 7.4; 5.4 dealt out).
+__device__ __forceinline__ void steal_ask(uint4* answer, unsigned long long* bar) {
+  const unsigned int b = (unsigned int)__cvta_generic_to_shared(bar);
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the last answer has been read
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], 16;" ::"r"(b) : "memory");
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(
+                   (unsigned int)__cvta_generic_to_shared(answer)),
+               "r"(b)
+               : "memory");
+}
+__device__ __forceinline__ bool steal_arrived(unsigned long long* bar, unsigned int phase) {
+  unsigned int ok;
+  asm volatile("{\n .reg .pred w;\n mbarrier.try_wait.parity.shared::cta.b64 w, [%1], %2;\n selp.u32 %0, 1, 0, w;\n}"
+               : "=r"(ok)
+               : "r"((unsigned int)__cvta_generic_to_shared(bar)), "r"(phase)
+               : "memory");
+  return ok != 0;
+}
+// the tile taken over, -1: none was left
+__device__ __forceinline__ int steal_answer(const uint4* answer) {
+  int tile;
+  asm volatile(
+      "{\n .reg .pred w;\n .reg .b128 h;\n ld.shared.b128 h, [%1];\n mov.u32 %0, -1;\n"
+      " clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 w, h;\n"
+      " @w clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %0, h;\n}"
+      : "=r"(tile)
+      : "r"((unsigned int)__cvta_generic_to_shared(answer))
+      : "memory");
+  return tile;
+}
+constexpr int kStealSpins = 1 << 22;   // polls of an answer, each up to some microseconds
+
 // Strided axes: thread (l, q) = q TL + l of a block owns chunk q of line
-// L0 + l (lanes on adjacent lines).  STAGED: a block takes several tiles of TL
-// lines in turn and copies the next tile's f into shared memory while it
-// solves the present one; otherwise a block has one tile and a thread loads its
-// rows straight into registers.  POW2: TL is a power of two (the division by any
-// other TL costs a block's start 2 %, FP32 epilogues 6-9 %).  THREADS: most
-// threads of a block, 512 or (FP32, 64 registers a thread) 1024.
-template <typename T, int R, bool PERIODIC, int EPI, bool STAGED, bool POW2, int THREADS>
+// L0 + l (lanes on adjacent lines).  STAGE: a block has one tile of TL lines and a
+// thread loads its rows straight into registers, or a block takes several tiles in
+// turn, by a fixed stride or dealt out, and copies the next tile's f into shared
+// memory while it solves the present one.  POW2: TL is a power of two (the
+// division by any other TL costs a block's start 2 %, FP32 epilogues 6-9 %).
+// THREADS: most threads of a block, 512 or (FP32, 64 registers a thread) 1024.
+template <typename T, int R, bool PERIODIC, int EPI, int STAGE, bool POW2, int THREADS>
 __global__ void __launch_bounds__(THREADS)
     ccd_chunk_strided_kernel(const __grid_constant__ CcdArgs a, const __grid_constant__ ChunkConst<T, R> K,
                              const T* __restrict__ gtab, int Q) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr bool STAGED = STAGE != kChunkDirect, STEAL = STAGE == kChunkSteal;
   const int t = threadIdx.x, TL = a.TL;
   const int q = POW2 ? t >> a.tl_shift : t * a.tl_inv >> 16, l = POW2 ? t & (TL - 1) : t - q * TL;
   T* G = reinterpret_cast<T*>(smem_raw);
@@ -417,7 +466,18 @@ __global__ void __launch_bounds__(THREADS)
   };
   int tile = blockIdx.x;
   int64_t base = base_of(tile);
-  if (STAGED) fetch(base);
+  __shared__ uint4 next_answer;
+  __shared__ __align__(8) unsigned long long next_bar;
+  unsigned int phase = 0;
+  if (STAGED) {
+    if (STEAL && t == 0) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((unsigned int)__cvta_generic_to_shared(&next_bar))
+                   : "memory");
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      steal_ask(&next_answer, &next_bar);
+    }
+    fetch(base);
+  }
   for (;;) {
     const bool act = q < Q && base >= 0;
     T fv[R + 2];
@@ -433,9 +493,26 @@ __global__ void __launch_bounds__(THREADS)
 #pragma unroll
       for (int i = 0; i < R + 2; ++i) fv[i] = T(0);
     }
-    const int next = tile + gridDim.x;
+    int next = tile + gridDim.x;
     int64_t nbase = -1;
-    if (STAGED && next < a.n_tiles) {
+    if constexpr (STEAL) {
+      bool in = false;
+      for (int spins = 0; spins < kStealSpins && !in; ++spins) in = steal_arrived(&next_bar, phase);
+      phase ^= 1u;
+      next = in ? steal_answer(&next_answer) : -1;
+      if (__syncthreads_or(!in)) {   // every thread has its rows, and the answer
+        // none came: these lines become NaN from end to end, and the block ends
+        // once the answer is in, or after as long again
+        fv[1] = T(NAN);
+        for (int spins = 0; spins < kStealSpins && !steal_arrived(&next_bar, phase ^ 1u); ++spins) {}
+        next = -1;
+      }
+      if (next >= 0) {
+        nbase = base_of(next);
+        fetch(nbase);
+        if (t == 0) steal_ask(&next_answer, &next_bar);
+      }
+    } else if (STAGED && next < a.n_tiles) {
       nbase = base_of(next);
       __syncthreads();   // every thread has its rows
       fetch(nbase);
@@ -443,7 +520,7 @@ __global__ void __launch_bounds__(THREADS)
     V2<T> x[R];
     chunk_solve<T, R, PERIODIC>(K, fv, q, Q, cnt, bl0, bl1, br0, br1, e, blockDim.x, t, TL, poison + l, G, x);
     if (act) chunk_store<T, R, PERIODIC, EPI>(a, K, x, base, inner, q, last, cnt, bl0, bl1, br0, br1);
-    if (!STAGED || next >= a.n_tiles) return;
+    if (!STAGED || (STEAL ? next < 0 : next >= a.n_tiles)) return;
     tile = next;
     base = nbase;
   }
