@@ -906,17 +906,16 @@ struct ChunkShape {
 //   20 are the better number on walls (321^3 221 with 20, 228 with 24, 242 with
 //   16; 385^3 the other way, 406 against 372) and 16 on periodic lines (321^3 198
 //   with 16, 209 with 20, 218 with 24; 320^3, aligned, 198 with 16, 178 with 24).
-// * FP32, d1 and d2 plainly stored: up to 1024 threads of 64 registers (a few
-//   spills on walls) instead of 512 of 74, where rows do not start on 16 bytes, so
-//   that short runs of them waste sectors, or a line has more than 64 chunks, of
-//   which 512 threads hold but 16 to 28 bytes of a row; again with several tiles
-//   per SM.  32 to 24 lines where two blocks fit, else the most that one holds
-//   (axis 0: 257^3 67 against 79, 273^3 93 against 108, 417^3 305 against 403,
-//   513^3 578 against 653, 1100 x 140 x 140 127 against 192, 2049 x 140 x 140 243
-//   against 387).  Elsewhere the spills cost more than the threads bring (340^3,
-//   aligned: 161 against 140; 193^3 in L2: 26 against 24), and so does the longer
-//   run on periodic lines whose rows lie close together (513^3 axis 1: 510
-//   against 469; axis 0, rows 1 MB apart: 536 against 570).
+// * FP32, plain, where there are several tiles per SM: up to 1024 threads of 64
+//   registers instead of 512 of 74; 32 to 24 lines where two blocks fit, else the
+//   most that one holds (wall, axis 0: 145^3 11.4 against 14.2, 209^3 34 against
+//   43, 257^3 66 against 79, 273^3 93 against 108, 300^3 87 against 103, 417^3 305
+//   against 403, 513^3 540 against 653, 1100 x 140 x 140 127 against 192, 2049 x
+//   140 x 140 243 against 387).  Not where rows start on 16 bytes and one block of
+//   32 lines leaves no room for a second (340^3 148 against 139).  Periodic lines,
+//   which take 64 registers anyway, only from 64 chunks on, where 512 threads hold
+//   but 16 to 28 bytes of a row, or where misaligned rows lie far apart (513^3 axis
+//   0, rows 1 MB apart: 536 against 570; axis 1 506 against 465, 256^3 50 against 44).
 // * Contiguous axis: 8 or 16 lines, whichever keeps more threads resident (193
 //   nodes: 45.3 with 8, 54.5 with 16; 162 nodes: 18.6 and 15.3).
 // * Fewer lines per block while that leaves half of the SMs without one, down
@@ -960,7 +959,7 @@ ChunkShape chunk_shape(const tpf_ccd_plan* p, bool contig, bool plain, bool heav
   };
   const bool wall = p->bc == TPF_BC_WALL, ragged = (inner * sizeof(T)) % 16 != 0;
   if (!F64 && !contig && plain &&
-      (Q > 64 || (ragged && (wall ? Q >= 14 : Q > 16 && inner * sizeof(T) >= 128 * 1024)))) {
+      (wall ? ragged || Q < 22 || Q > 32 : Q > 64 || (ragged && Q > 16 && inner * sizeof(T) >= 128 * 1024))) {
     int tl = 0;
     for (int k : {24, 28, 32})   // two blocks of an SM's 1024 threads
       if (k * Q <= 512) tl = k;
