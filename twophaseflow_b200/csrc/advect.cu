@@ -493,9 +493,14 @@ __global__ void compression_flux_kernel(CompArgs a) {
 // ('periodic': g[n-2] left, g[1] right) or the end node itself ('neumann',
 // 'outflow') (filtered_divergence, reinit_ops.py:83-105; pad_ghost_cells,
 // core/boundary.py:249-292).
-// 193^3 FP64: 39.9 us with a 64-bit division and remainder per node, 33.4 with AxisCoord.
+// The grid is the blocks that are resident at once, 8 per SM at 32 registers: with
+// 34 to 38 only 6 were, and of 16 per SM launched the last ones ran through
+// the array a second time, which fields beyond L2 felt once the coordinate was
+// cheap (64-bit division and remainder per node, then AxisCoord, then this; us,
+// accumulated, axis 0): FP32 300^3 162, 210, 128; 257^3 98, 121, 81; FP64 300^3
+// 157, 142, 115; 193^3 40.6, 35.1, 31.9.
 template <typename T>
-__global__ void filtered_div_kernel(int64_t tot, tpf::AxisCoord pos, int pad, double eps_d, const T* g,
+__global__ void __launch_bounds__(256, 8) filtered_div_kernel(int64_t tot, tpf::AxisCoord pos, int pad, double eps_d, const T* g,
                                     const double* J, int accumulate, T* div) {
   const int64_t n = pos.n, inner = pos.inner;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < tot; i += (int64_t)gridDim.x * blockDim.x) {
@@ -782,11 +787,11 @@ static int filtered_divergence_axis(int ndim, const int64_t* shape, int axis, in
   const tpf::AxisCoord pos(outer, n, inner);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (dtype == TPF_F64)
-    filtered_div_kernel<double><<<blocks_for(tot, 16), 256, 0, st>>>(tot, pos, pad, eps_d,
+    filtered_div_kernel<double><<<blocks_for(tot, 8), 256, 0, st>>>(tot, pos, pad, eps_d,
                                                                     static_cast<const double*>(g), J, accumulate,
                                                                     static_cast<double*>(div));
   else
-    filtered_div_kernel<float><<<blocks_for(tot, 16), 256, 0, st>>>(tot, pos, pad, eps_d,
+    filtered_div_kernel<float><<<blocks_for(tot, 8), 256, 0, st>>>(tot, pos, pad, eps_d,
                                                                    static_cast<const float*>(g), J, accumulate,
                                                                    static_cast<float*>(div));
   TPF_CUDA_TRY(cudaGetLastError());
