@@ -83,3 +83,63 @@ def test_batch_of_any_make_up(cuda_device, shapes, precision):
         one = s.solve(rhs[k], rho[k])
         scale = float(one.abs().max())
         assert float((got[k] - one).abs().max()) <= bar * scale, k
+
+
+def _exact(grid, rho, rhs, pin):
+    """The pinned system's solution beyond 64 bits: factorized in them, residuals of the flux form in extended precision."""
+    import scipy.sparse as sp
+    import scipy.sparse.linalg as spla
+    c = [np.asarray(x, dtype=np.float64) for x in grid.coords]
+    d = [np.diff(x) for x in c]
+    dv = [np.concatenate([x[:1] / 2, (x[1:] + x[:-1]) / 2, x[-1:] / 2]) for x in d]
+    s = [2 / (rho[:-1] + rho[1:]) / d[0][:, None] * dv[1], 2 / (rho[:, :-1] + rho[:, 1:]) / d[1] * dv[0][:, None]]
+    idx = np.arange(rho.size).reshape(rho.shape)
+    i, j = (np.concatenate(x) for x in ((idx[:-1].ravel(), idx[:, :-1].ravel()), (idx[1:].ravel(), idx[:, 1:].ravel())))
+    s = np.concatenate([x.ravel() for x in s])
+    b = -(rhs * dv[0][:, None] * dv[1]).ravel()
+    b[pin] = 0.0
+    diag = np.zeros(rho.size)
+    np.add.at(diag, i, s)
+    np.add.at(diag, j, s)
+    diag[pin] = 1.0
+    on = (i != pin) & (j != pin)
+    a = sp.coo_matrix((np.concatenate([-s[on], -s[on], diag]),
+                       (np.concatenate([i[on], j[on], idx.ravel()]), np.concatenate([j[on], i[on], idx.ravel()]))))
+    lu = spla.splu(a.tocsc())
+    x = np.zeros(rho.size, np.longdouble)
+    for _ in range(5):
+        flux = s.astype(np.longdouble) * (x[i] - x[j])
+        r = b.astype(np.longdouble)
+        np.add.at(r, i, -flux)
+        np.add.at(r, j, flux)
+        r[pin] = 0.0
+        x += lu.solve(r.astype(np.float64))
+        x[pin] = 0.0
+    return x.reshape(rho.shape)
+
+
+@pytest.mark.parametrize("trial", [0, 1])
+def test_batch_against_the_exact_solution(cuda_device, trial):
+    """Sixteen systems to 1e-10, in one launch and one by one, against their
+    solutions beyond 64 bits: the error is A^-1 of a residual of 1e-10 of the
+    right-hand side, a few 1e-11 of max|p| on these systems, and at most 1e-10."""
+    import torch
+    from twophaseflow_b200 import PPESolverFVMMatrixFree, UniformGrid, solve_batched
+
+    class Cfg:
+        pseudo_tol = 1e-10
+        pseudo_maxiter = 200000
+        ppe_iteration_method = "cg"
+        ppe_preconditioner = "jacobi"
+
+    rng = np.random.default_rng(trial)
+    shapes = [tuple(int(n) for n in rng.integers(48, 97, 2)) for _ in range(16)]
+    solvers = [PPESolverFVMMatrixFree(None, Cfg(), UniformGrid(N)) for N in shapes]
+    rho = [droplet_density(N, n_drops=3, rho_g=1e-2, seed=100 * trial + k) for k, N in enumerate(shapes)]
+    rhs = [divergence_rhs(N, seed=1000 + 100 * trial + k) for k, N in enumerate(shapes)]
+    rho_d, rhs_d = ([torch.from_numpy(a).to(cuda_device) for a in x] for x in (rho, rhs))
+    got = solve_batched(solvers, rhs_d, rho_d)
+    for k, s in enumerate(solvers):
+        exact = _exact(s.grid, rho[k], rhs[k], s._pin_dof)
+        for p in (got[k], s.solve(rhs_d[k], rho_d[k])):
+            assert np.abs(p.cpu().numpy() - exact).max() <= 1e-10 * np.abs(exact).max(), shapes[k]
