@@ -279,8 +279,8 @@ def time_ccd(N, bc, axis, dtype="f64", reps=10):
 
 
 # DRAM bytes read + written by one cg1_band_kernel solve at 513^2 (ncu,
-# dram__bytes_read.sum + dram__bytes_write.sum of the launch)
-PCG_BAND_DRAM_BYTES_PER_SOLVE = 11.5e6
+# dram__bytes_read.sum + dram__bytes_write.sum of the launch; profiles/cg1_band_kernel_512.md)
+PCG_BAND_DRAM_BYTES_PER_SOLVE = 11.7e6
 # DRAM bytes of one smooth_block_kernel launch (4 sweeps) at 513^2 (ncu,
 # cold caches: the five inputs read once; the output stays in L2)
 SMOOTH_DRAM_BYTES_PER_LAUNCH = 10.5e6

@@ -9,8 +9,9 @@
 // Riccati recurrence), so the two sweeps are constant-coefficient recurrences
 //     y_j = b_j + A y_{j-1},   x_j = P y_j + B x_{j+1},   A = -Lf, B = -H,
 // whose powers decay like 0.455^k.  Hence a chunk needs only the end values of
-// the kChunkWindow chunks next to it (0.455^64 = 1e-22 of the carry is left
-// out): a thread sweeps its chunk from a zero carry, publishes the end value,
+// the kChunkWindow chunks next to it: what is left out is 0.455^64 = 1e-22 of the
+// carry, on a ring whose last chunk is short at most 0.455^49 = 2e-17 (that chunk
+// counts as one of the window's).  A thread sweeps its chunk from a zero carry, publishes the end value,
 // reads its neighbours', and sweeps again from the carry they add up to.  No
 // scan over the line, no per-row tables.  (Adding A^(r+1) times the carry to
 // row r instead of the second sweep takes as many multiplications, but each
@@ -29,9 +30,11 @@
 // per axis in FP32 at 192 x 161 x 226); at 128 registers a thread 16 warps are
 // resident per SM, and between the two barriers they issue in 44 % of the
 // cycles, 430 FP64 instructions a warp and tile.  8 rows a thread and twice the
-// warps (64 registers) is slower, 182 us.  Against the kernels this replaces, a
-// thread per line that read f twice and a scan of 2 x 2 maps over the warps of
-// a line (us per call): 257^3 FP64 wall 99 / 99 / 97 on axes 0 / 1 / 2, before
+// warps (64 registers) is slower, 160-180 us.  The FP64 wall kernels of the
+// corrector and the variable-density term spill 16 to 48 bytes of a thread's
+// stack at their 128 registers; the others spill nothing.  Against the kernels
+// this replaces, a thread per line that read f twice and a scan of 2 x 2 maps over
+// the warps of a line (us per call): 257^3 FP64 wall 99 / 99 / 97 on axes 0 / 1 / 2, before
 // 116 / 118 / 209; periodic 96 / 95 / 91, before 105 / 108 / 193; FP32 192 x 161
 // x 226 19 / 17 / 24, before 31 / 32 / 80; 129 x 97 x 162 13 / 13 / 15, before
 // 64 / 80 / 51; 1025^2 8.7 / 9.2, before 25 / 22.

@@ -1310,7 +1310,7 @@ __device__ __forceinline__ void cg1_band_mixed_body(const BandArgs& a, const int
 // any fence.  Only w of the edge nodes travels: the reader carries their r and
 // s itself by the same two recurrences (fused multiply-adds spelled out, so
 // both copies have the same bits).
-// 513^2 to 1e-8: 25.6 -> 11.6 ms, 3.0 us an iteration, of which ~1.5 us are
+// 513^2 to 1e-8: 25.6 -> 11.6 ms, 3.15 us an iteration, of which ~1.5 us are
 // the exchange over 148 blocks alone.
 //
 // 256 threads of up to 255 registers rather than 512 of 128: the per-warp cost
@@ -1320,7 +1320,9 @@ __device__ __forceinline__ void cg1_band_mixed_body(const BandArgs& a, const int
 // two neighbours along the row mostly are its own registers; E is odd, which
 // keeps the E-strided shared-memory accesses free of bank conflicts.  Up to
 // E = 9 the couplings are in registers too (x from E = 9 on in shared memory);
-// E = 11 keeps them in shared memory.  E is the smallest that covers the
+// E = 11 keeps them in shared memory.  Not all of it fits the 255 registers: E = 7
+// (which runs 513^2) spills 118 bytes on stores and 132 on loads, E = 9 178 and
+// 252, E = 11 44 and 44, smaller ones nothing.  E is the smallest that covers the
 // largest range, so small systems do not iterate over empty slots.
 constexpr int kBandMaxE = 11;       // nodes per thread: 2 816 per SM, 416 768 per 148 SMs (645^2)
 constexpr int kBandCregE = 9;       // up to here the couplings are in registers too
