@@ -287,3 +287,26 @@ def test_epilogues_of_the_contiguous_axis_cost_their_bytes(cuda_device, dtype):
             best.append(a.elapsed_time(b))
         times[kind] = min(best)
     assert times["vd"] <= 1.5 * 5 / 3 * times["plain"], times
+
+
+def test_dealt_out_tiles_beside_other_launches(cuda_device):
+    """Two streams of calls whose tiles are dealt out, their blocks resident
+    beside each other's and taken over as they wait: every call has the bits of
+    one that runs by itself."""
+    import torch
+    from twophaseflow_b200 import CCDSolver, UniformGrid
+    shapes = [(1025, 130, 131), (1340, 97, 75)]
+    streams = [torch.cuda.Stream() for _ in shapes]
+    fields = [torch.randn(s, device=cuda_device, dtype=torch.float64) for s in shapes]
+    solvers = [CCDSolver(UniformGrid(tuple(n - 1 for n in s)), None, bc_type="wall") for s in shapes]
+    alone = [c.differentiate(f, 0) for c, f in zip(solvers, fields)]
+    torch.cuda.synchronize()
+    results = [[], []]
+    for _ in range(6):
+        for k in range(2):
+            with torch.cuda.stream(streams[k]):
+                results[k].append(solvers[k].differentiate(fields[k], 0))
+    torch.cuda.synchronize()
+    for k in range(2):
+        for d in results[k]:
+            assert torch.equal(d[0], alone[k][0]) and torch.equal(d[1], alone[k][1])
